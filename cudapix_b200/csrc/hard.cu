@@ -18,7 +18,20 @@
 // to k_hard_leaves with a snapshot of the sub-segment, (3) crosses off p_b,
 // counting cleared bits and keeping the counters current.  The level
 // parameters (x/p, candidate range, first multiple) are computed 32 levels at
-// a time, one level per lane, and broadcast by shuffles.  Every 32 levels the
+// a time, one level per lane, and broadcast by shuffles.
+//
+// Blocks of 32 levels whose primes have few multiples in a sub-segment (and no
+// leaf set for k_hard_leaves) go through at once instead: cross_levels takes
+// one multiple of each level a step, the block's candidates are walked as one
+// sequence, and each leaf is counted on the bitmap after the whole block plus
+// the bits up to u that its own and higher levels cleared, which cross_levels
+// notes down.  One level at a time such a level costs a warp some 250 issue
+// slots for a handful of multiples and one or two leaves, with most lanes
+// idle: integer issue bounds the kernel (81% of the slots), not memory.
+// On a B200: the sieve of pi(1e15) 2.82 -> 2.15 ms, of pi(1e17) 26.4 -> 20.1,
+// of pi(2e19) 1308 -> 904, of pi(1e12) 0.279 -> 0.184.
+//
+// Every 32 levels the
 // CTA combines its warps: carries between sub-segments enter the hard sum and
 // the per-segment (count, Sum(-mu)) pairs go to k_hard_combine, which adds the
 // carries between segments.
@@ -28,9 +41,17 @@
 #include <algorithm>
 #include <mutex>
 
-#include "sieve.cuh"
+#include "levels.cuh"
 
 namespace cpx {
+
+// A block of 32 levels is crossed off at once (cross_levels) when its smallest
+// prime has at most this many multiples in a warp's sub-segment.  Below that
+// the bits a block clears outnumber the leaves it answers, and each leaf is
+// compared with all of them.  On a B200 the sieve of pi(1e15) took 2.82 ms one
+// level at a time and 2.52 / 2.15 / 2.59 with 8 / 16 / 32 here; of pi(2e19)
+// 1308 and 929 / 904 / 888.
+constexpr uint32_t kLevelWindows = 16;
 
 template <class XT>
 __global__ void __launch_bounds__(512, 2) k_hard(const QD *__restrict__ qd, uint32_t Q,
@@ -78,12 +99,14 @@ __global__ void __launch_bounds__(512, 2) k_hard(const QD *__restrict__ qd, uint
     o += ((Lmax / 128) + 15) & ~size_t(15);
     uint32_t *loff = reinterpret_cast<uint32_t *>(sp + o);  // [NW][32] lane prefixes
     o += T * 4;
-    LvlOut *area = reinterpret_cast<LvlOut *>(sp + o);      // [2][NW][32]
-    o += 2 * NW * 32 * sizeof(LvlOut);
+    LvlSum *area = reinterpret_cast<LvlSum *>(sp + o);      // [2][NW][32]
+    o += 2 * NW * 32 * sizeof(LvlSum);
     o = (o + 15) & ~size_t(15);
     i128 *s_red = reinterpret_cast<i128 *>(sp + o);
     o += 32 * sizeof(i128);
     uint32_t *lbuf = reinterpret_cast<uint32_t *>(sp + o) + kLeafBuf * warp;  // this warp's gathered leaves
+    o += NW * kLeafBuf * 4;
+    uint32_t *ev = reinterpret_cast<uint32_t *>(sp + o) + kEvCap * warp;      // this warp's cleared bits
     uint32_t *wl = loff + 32 * warp;  // this warp's lane prefixes
 
     const uint32_t c0 = CPT * tid;  // first owned chunk (of the segment)
@@ -113,7 +136,151 @@ __global__ void __launch_bounds__(512, 2) k_hard(const QD *__restrict__ qd, uint
         // levels of the block with candidates in the sub-segment (most levels of
         // the high segments have none: they only cross off)
         const unsigned act = __ballot_sync(FULL, lane < nl && lv.mhi > lv.mlo);
-        LvlOut mine = {0, 0, 0xFFFFFFFFu, 0};
+        LvlSum mine = {0, 0, 0xFFFFFFFFu};
+        LvlSum *ar = area + (grp & 1) * NW * 32;
+        // table entries of each level's candidates: pi-table words of the
+        // prime-only levels, 4-m groups of packed mu*lpf of the others
+        const bool prime_j = (uint64_t)lp * lp > y;
+        const uint32_t qa_j = lmlo > lp ? lmlo : lp;
+        uint32_t nw_j = 0, ng_j = 0;
+        if (lane < nl && lmhi > lmlo) {
+            if (!prime_j) ng_j = ((lmhi - 1) >> 3) - ((lmlo + 1) >> 3) + 1;
+            else if (lmhi > qa_j) nw_j = ((lmhi - 1) >> 7) - (qa_j >> 7) + 1;
+        }
+        const bool heavy_j = max_jobs && offload_min && 8 * nw_j + 4 * ng_j >= offload_min;
+        const uint32_t pmin = __shfl_sync(FULL, lp, 0);
+        if ((uint64_t)pmin * kLevelWindows >= Lw && !__any_sync(FULL, heavy_j)) {
+            // ---- the block's levels at once
+            const bool leaves = __any_sync(FULL, (nw_j | ng_j) != 0);
+            uint32_t i = li0, w_end = pmin, cleared = 0;
+            ar[warp * 32 + lane].ms = 0;
+            if (!leaves) {
+                cross_levels<false>(bm, cnt8, lp, i, pmin, w_end, cleared, s, CPT * 32 * warp, lane, Lw, ev, 0);
+            } else {
+                uint2 *lb2 = reinterpret_cast<uint2 *>(lbuf);
+                constexpr uint32_t kCap2 = kLeafBuf / 2;
+                uint32_t ex_w, ex_g;
+                const uint32_t tot_w = warp_place(nw_j, lane, ex_w), tot_g = warp_place(ng_j, lane, ex_g);
+                uint32_t k_lo = 0;  // the slice's leaves have their counts' bits [0, kk), k_lo < kk <= k_hi
+                for (;;) {
+                    // cleared bits of the earlier slices at this lane's level and above
+                    uint32_t suf = cleared;
+#pragma unroll
+                    for (int oo = 1; oo < 32; oo <<= 1) {
+                        const uint32_t t = __shfl_down_sync(FULL, suf, oo);
+                        if (lane + oo < 32) suf += t;
+                    }
+                    const uint32_t nev = cross_levels<true>(bm, cnt8, lp, i, pmin, w_end, cleared, s, CPT * 32 * warp,
+                                                            lane, Lw, ev, kEvCap);
+                    const uint32_t k_hi = min(w_end - pmin, Lw);
+                    if (lane < 4 && nev + lane < kEvCap) ev[nev + lane] = kEvMask;  // the last four events
+                    // lane prefixes of the sub-segment from the chunk counters
+                    uint32_t off0;
+                    warp_place(counter_sum(cnt8 + c0, CPT), lane, off0);
+                    wl[lane] = off0;
+                    uint32_t nbuf = 0;
+                    // Answers the gathered leaves (m, level k | (mu(m) = -1) << 31): the
+                    // survivors of level b - 1 up to u are those after the whole block
+                    // and the bits up to u that levels b and above took.
+                    auto flush = [&] {
+                        __syncwarp();
+                        for (uint32_t j0 = 0; j0 < nbuf; j0 += 32) {
+                            const bool on = j0 + lane < nbuf;
+                            uint2 e = make_uint2(1, 0);
+                            if (on) e = lb2[j0 + lane];
+                            const uint32_t key = e.y & 31u;
+                            XT xk;
+                            if (sizeof(XT) == 8) {
+                                xk = (XT)__shfl_sync(FULL, (unsigned long long)lxp, key);
+                            } else {
+                                const unsigned long long a0 = __shfl_sync(FULL, (unsigned long long)lxp, key);
+                                const unsigned long long a1 =
+                                    __shfl_sync(FULL, (unsigned long long)((u128)lxp >> 64), key);
+                                xk = (XT)(((u128)a1 << 64) | a0);
+                            }
+                            uint32_t cv = __shfl_sync(FULL, suf, key);
+                            if (on) {
+                                const uint64_t uu = leaf_quot(xk, (double)(uint64_t)xk, e.x, q41);
+                                const uint32_t kk = ((uint32_t)uu - (uint32_t)lo_w + 1u) >> 1;
+                                if (kk <= k_hi && (kk > k_lo || !k_lo)) {
+                                    cv += sub_count(uu);
+                                    const uint32_t kmin = key << kEvBit;
+                                    for (uint32_t t = 0; t < nev; t += 4) {
+                                        const uint4 v = *reinterpret_cast<const uint4 *>(ev + t);
+                                        cv += (v.x >= kmin && (v.x & kEvMask) < kk) + (v.y >= kmin && (v.y & kEvMask) < kk) +
+                                              (v.z >= kmin && (v.z & kEvMask) < kk) + (v.w >= kmin && (v.w & kEvMask) < kk);
+                                    }
+                                    const bool plus = (e.y >> 31) != 0;
+                                    if (plus) S += cv;
+                                    else S -= cv;
+                                    atomicAdd(&ar[warp * 32 + key].ms, plus ? 1 : -1);
+                                }
+                            }
+                        }
+                        __syncwarp();
+                        nbuf = 0;
+                    };
+                    for (uint32_t base = 0; base < tot_w; base += 32) {
+                        const uint32_t f = base + lane;
+                        const uint32_t jq = item_owner(ex_w, f);
+                        const uint32_t exq = __shfl_sync(FULL, ex_w, jq);
+                        const uint32_t qaq = __shfl_sync(FULL, qa_j, jq), mhq = __shfl_sync(FULL, lmhi, jq);
+                        uint64_t qb = 0, wq = 0;
+                        if (f < tot_w) {
+                            wq = (qaq >> 7) + (f - exq);
+                            qb = __ldg(reinterpret_cast<const ulonglong2 *>(Tpi) + wq).x & range_mask(wq, qaq, mhq);
+                        }
+                        // dense rounds (over 128 leaves) go in halves and quarters of a word
+                        for (uint32_t part = 0; __any_sync(FULL, qb != 0); part++) {
+                            uint64_t now = qb;
+                            if (__reduce_add_sync(FULL, (uint32_t)__popcll(qb)) > kCap2) now = qb & (0xFull << (4 * part));
+                            qb &= ~now;
+                            uint32_t off;
+                            const uint32_t tot_r = warp_place((uint32_t)__popcll(now), lane, off);
+                            if (nbuf + tot_r > kCap2) flush();
+                            uint32_t kk = nbuf + off;
+                            while (now) {
+                                const int j = __ffsll((long long)now) - 1;
+                                now &= now - 1;
+                                lb2[kk++] = make_uint2((uint32_t)(128 * wq + 2 * j + 1), jq | 0x80000000u);
+                            }
+                            nbuf += tot_r;
+                        }
+                    }
+                    for (uint32_t base = 0; base < tot_g; base += 32) {
+                        const uint32_t f = base + lane;
+                        const uint32_t jq = item_owner(ex_g, f);
+                        const uint32_t exq = __shfl_sync(FULL, ex_g, jq), pq = __shfl_sync(FULL, lp, jq);
+                        const uint64_t mlq = __shfl_sync(FULL, lmlo, jq), mhq = __shfl_sync(FULL, lmhi, jq);
+                        const uint64_t i_lo = (mlq + 1) >> 1, i_hi = (mhq - 1) >> 1;
+                        uint32_t neg = 0, vm = 0;
+                        uint64_t g4 = 0;
+                        if (f < tot_g) {
+                            g4 = (i_lo >> 2) + (f - exq);
+                            vm = valid_group(__ldg(reinterpret_cast<const int4 *>(MU) + g4), g4, i_lo, i_hi, pq, &neg);
+                        }
+                        uint32_t off;
+                        const uint32_t tot_r = warp_place((uint32_t)__popc(vm), lane, off);
+                        if (nbuf + tot_r > kCap2) flush();
+                        uint32_t kk = nbuf + off;
+                        while (vm) {
+                            const int kq = __ffs(vm) - 1;
+                            vm &= vm - 1;
+                            lb2[kk++] = make_uint2((uint32_t)(2 * (4 * g4 + kq) + 1), jq | (((neg >> kq) & 1u) << 31));
+                        }
+                        nbuf += tot_r;
+                    }
+                    flush();
+                    if (k_hi == Lw) break;
+                    k_lo = k_hi;
+                }
+            }
+            uint32_t before;
+            const uint32_t all = warp_place(cleared, lane, before);
+            mine.cnt = tot - before;
+            tot -= all;
+            mine.ms = ar[warp * 32 + lane].ms;
+        } else
         for (uint32_t k = 0; k < nl; k++) {
             const uint32_t b = gb + k;
             const uint32_t p = __shfl_sync(FULL, lp, k);
@@ -270,7 +437,6 @@ __global__ void __launch_bounds__(512, 2) k_hard(const QD *__restrict__ qd, uint
             }
         }
         // ---- combine the warps of the CTA for these 32 levels
-        LvlOut *ar = area + (grp & 1) * NW * 32;
         ar[warp * 32 + lane] = mine;
         __syncthreads();
         if (warp == 0 && lane < nl) {
@@ -278,7 +444,7 @@ __global__ void __launch_bounds__(512, 2) k_hard(const QD *__restrict__ qd, uint
             uint64_t carry = 0;
             int32_t msum = 0;
             for (uint32_t w = 0; w < NW; w++) {
-                const LvlOut e = ar[w * 32 + lane];
+                const LvlSum e = ar[w * 32 + lane];
                 Sx += (i128)carry * e.ms;
                 if (e.job != 0xFFFFFFFFu) jobs[e.job].carry = carry;
                 carry += e.cnt;
@@ -532,7 +698,7 @@ size_t hard_snapshot_stride(uint32_t lbits_sub) { return snap_stride(lbits_sub);
 size_t hard_smem_bytes(uint32_t lbits, uint32_t threads, bool wide)
 {
     (void)wide;
-    return hard_smem(lbits, threads);
+    return levels_smem(lbits, threads);
 }
 
 void launch_hard_leaves(cpx_ctx *ctx, const Plan &pl, uint32_t lbits_sub)
@@ -557,7 +723,7 @@ template <class XT> static void hard_go(cpx_ctx *ctx, const Plan &pl)
     CPX_LAUNCH("k_hard_plan");
     note_launch(ctx);
     scan_u64(ctx, pl.seg_off, pl.n_seg);
-    const size_t smem = hard_smem(pl.lbits_max, pl.hard_threads);
+    const size_t smem = levels_smem(pl.lbits_max, pl.hard_threads);
     const uint32_t lbits_sub = pl.lbits_max - (uint32_t)(__builtin_ctz(pl.hard_threads) - 5);
     if (pl.time_hard) CPX_CUDA(cudaEventRecord(ctx->ev_hard0, ctx->stream));
     if (pl.max_jobs) {
@@ -591,7 +757,7 @@ template <class XT> static void hard_go(cpx_ctx *ctx, const Plan &pl)
 void prepare_hard(cpx_ctx *ctx, const Plan &pl)
 {
     if (!pl.n_seg) return;
-    const size_t smem = hard_smem(pl.lbits_max, pl.hard_threads);
+    const size_t smem = levels_smem(pl.lbits_max, pl.hard_threads);
     if (smem > ctx->smem_optin) fail(CPX_EINVAL, "hard-leaf segment needs more shared memory than a block can have");
     static std::mutex m;
     static int done_dev[2] = {-1, -1};
