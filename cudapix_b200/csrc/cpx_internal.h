@@ -96,6 +96,7 @@ struct cpx_ctx {
     cpx::DevBuf b_flush;     // L2 flush buffer (bench only)
     cpx::DevBuf b_jobs, b_jobctl, b_snap;  // offloaded hard-leaf sets and their snapshots
     cpx::DevBuf b_levels;                  // per-level records of a part of a split query
+    cpx::DevBuf b_lvpar;                   // per-level constants of the lone-query sieve
     unsigned long long *d_acc = nullptr;  // per-query accumulators (grown)
     size_t acc_cap = 0;
     unsigned long long *h_acc = nullptr;  // pinned mirror
@@ -113,7 +114,7 @@ struct cpx_ctx {
     uint32_t hard_log2_bits = 18;  // hard-leaf segment size (odd numbers, bits)
     uint32_t hard_threads = 256;
     bool hard_params_set = false;      // cpx_set_hard_params was called (no size rule then)
-    uint32_t hard_offload_min = 1024;  // candidates of a (sub-segment, level) sent to k_hard_leaves
+    uint32_t hard_offload_min = 1024;  // candidates of a (sub-segment, level) sent to k_hard_leaves (shared sieve)
     uint32_t hard_shared = 1;          // batch-shared sieve: 0 never, 1 batches, 2 always
     uint32_t hard_persist = 1;         // shared sieve as a persistent launch over a unit queue
     uint64_t hard_offload_bytes = 4ull << 30;  // snapshot pool budget of one batch

@@ -112,8 +112,8 @@ static uint64_t segments_at_level(u128 x, uint64_t span, uint64_t p, uint64_t se
     return hi >= first ? hi - first + 1 : 0;
 }
 
-// Number of (sub-segment, level) leaf sets of one query that k_hard hands to
-// k_hard_leaves at threshold thr: the same candidate bounds as k_hard's warps
+// Number of (sub-segment, level) leaf sets of one query that the shared sieve
+// hands to k_hard_leaves at threshold thr: the same candidate bounds as its warps
 // (m in (max(y/p, xp/hi_w), min(y, xp/lo_w, x/p^3)], prime m only when
 // p^2 > y).  Along a level the candidate count rises while the sub-segments
 // reach into the leaves' smallest u and falls once xp/lo_w is the upper
@@ -328,6 +328,92 @@ void merge_hard_part(std::vector<u128> &carry, i128 &H, const HardLevel *rec, ui
     }
 }
 
+// About how many hard leaves of a query lie in [lo, hi), from a sample of the
+// nlv levels; only how the work is split depends on it.
+static double leaf_estimate(const QD &d, const std::vector<uint32_t> &hP, uint32_t c, double lo, double hi, uint32_t nlv)
+{
+    const double x = (double)d.x, y = (double)d.y;
+    const uint32_t ns = std::min<uint32_t>(nlv, 12);
+    double sum = 0.0;
+    uint64_t i0 = 0;
+    for (uint32_t k = 1; k <= ns; k++) {
+        const uint64_t i1 = std::max<uint64_t>(i0 + 1, (uint64_t)nlv * k * k / ((uint64_t)ns * ns));
+        const double p = hP[c + (i0 + i1) / 2], xp = x / p;
+        const double mlo = std::max(y / p, xp / hi);
+        const double mhi = std::min(std::min(y, xp / (p * p)), lo > 0 ? xp / lo : y);
+        if (mhi > mlo) {
+            const double first = p * p > y ? std::max(mlo, p) : mlo;
+            if (mhi > first) sum += (double)(i1 - i0) * (mhi - first) / std::log(p * p > y ? mhi : p);
+        }
+        i0 = i1;
+        if (i0 >= nlv) break;
+    }
+    return sum;
+}
+
+// The units before each of the first segments whose leaves take more time than
+// the rest of a unit (k_hard): such a segment's leaves are split over several
+// units, each of which sieves the segment again.  A unit costs each of its
+// warps about 600 issue slots for each of the first 64 levels and 80 for each
+// of the others, a leaf kLeafSlots.  A unit should
+// not take more than about half of a resident CTA's share of the whole query
+// either (the first segments start first, and the rest fills in behind them).
+constexpr double kLeafSlots = 5.0;
+static void dense_units(const QD &d, const std::vector<uint32_t> &hP, uint32_t c, uint32_t threads, uint32_t ctas,
+                        std::vector<uint32_t> &base)
+{
+    base.clear();
+    const uint64_t span = 2ull << d.lbits;
+    const double nw = threads / 32;
+    auto levels = [&](uint64_t seg) -> uint32_t {  // seg_levels of the device, at most
+        const uint64_t lo = seg * span, hi = lo + span;
+        uint64_t v = d.r4;
+        if (lo) v = std::min<uint64_t>(v, cpx_isqrt((u128)((d.x - 1) / lo)));
+        v = std::min<uint64_t>(v, cpx_isqrt((u128)(hi - 1)));
+        const uint64_t n = (uint64_t)(std::upper_bound(hP.begin(), hP.begin() + d.nb, v,
+                                                       [](uint64_t a, uint32_t b) { return a < b; }) -
+                                      hP.begin());
+        return n > c ? (uint32_t)(n - c) : 0;
+    };
+    struct Pt {
+        uint64_t seg;
+        double leaf, fixed;
+    };
+    std::vector<Pt> pts;
+    double total = 0.0;
+    for (uint64_t k = 0; k < d.nseg;) {
+        const uint64_t n = k < 16 ? 1 : k / 8;
+        const uint32_t nlv = levels(d.seg0 + k);
+        Pt t{k, 0.0, 0.0};
+        if (nlv) {
+            // the leaves of the segment's densest sub-segment (its first, or in the
+            // segment where the leaves begin its last) set the CTA's time
+            const double lo = (double)(d.seg0 + k) * (double)span, sub = (double)span / nw;
+            double lf = leaf_estimate(d, hP, c, lo, lo + sub, nlv);
+            if (k < 16) lf = std::max(lf, leaf_estimate(d, hP, c, lo + span - sub, lo + (double)span, nlv));
+            t.leaf = kLeafSlots * nw * lf;
+            t.fixed = nw * (std::min(nlv, 64u) * 600.0 + (nlv > 64 ? nlv - 64 : 0) * 80.0);
+        }
+        total += (double)std::min<uint64_t>(n, d.nseg - k) * (t.leaf + t.fixed);
+        pts.push_back(t);
+        k += n;
+    }
+    const double share = 0.5 * total / ctas;
+    std::vector<uint32_t> parts;
+    size_t last = 0;  // segments up to the last one with several units
+    for (size_t j = 0; j < pts.size() && pts[j].seg < (1u << 16); j++) {
+        const uint64_t end = j + 1 < pts.size() ? pts[j + 1].seg : d.nseg;
+        const double unit = std::max(pts[j].fixed, share);
+        const uint32_t n = unit > 0 ? (uint32_t)std::min(64.0, std::ceil(pts[j].leaf / unit)) : 1;
+        if (n >= 2) last = end;
+        parts.resize(end, std::max(n, 1u));
+    }
+    if (!last) return;
+    base.resize(last + 1);
+    base[0] = 0;
+    for (size_t k = 0; k < last; k++) base[k + 1] = base[k] + parts[k];
+}
+
 constexpr uint64_t kWindowBytes = 32ull << 30;
 constexpr uint64_t kWindowEntries = 1ull << 31;
 
@@ -535,8 +621,8 @@ void compute_needs(const BatchReq &rq, std::vector<QD> &qd, TableNeed &need, boo
         if (mask & TERM_EASY) N = std::max<uint64_t>(N, std::max(sx, y) + 1);
         if (mask & (TERM_ORD | TERM_HARD)) Y = std::max(Y, y);
         if (mask & TERM_HARD) {
-            Pneed = std::max<uint64_t>(Pneed, r4 + 1);
-            // carries below p_b^2 come from the pi table; prime m of the sparse levels from its bitmap
+            Pneed = std::max<uint64_t>(Pneed, std::max(r4, y) + 1);  // and the prime m of the prime-only levels
+            // carries below p_b^2 and the ranks of the prime m come from the pi table
             N = std::max<uint64_t>(N, std::max<uint64_t>(r4 * r4 + 2, y + 1));
         }
         if (mask & TERM_EASY) {
@@ -730,7 +816,8 @@ replan:  // again without the batch alpha when its shared sieve would not fit (b
     std::vector<uint64_t> pre(6 * (size_t)(Q + 1), 0);
     uint64_t *p_ord = pre.data(), *p_p2 = p_ord + (Q + 1), *p_triv = p_p2 + (Q + 1), *p_easy = p_triv + (Q + 1),
              *p_seg = p_easy + (Q + 1), *p_comb = p_seg + (Q + 1);
-    std::vector<uint64_t> q_ent(Q, 0);
+    std::vector<uint64_t> q_ent(Q, 0), q_rows(Q, 0);
+    std::vector<std::vector<uint32_t>> q_dense(shared || !(mask & TERM_HARD) ? 0 : Q);
     const size_t nblk = (Q + kPlanBlock - 1) / kPlanBlock;
     std::vector<std::vector<EasyLvl>> blk_elv(nblk);
     std::vector<uint64_t> blk_ecomp(nblk, 0);
@@ -795,10 +882,25 @@ replan:  // again without the batch alpha when its shared sieve would not fit (b
                     }
                     n_seg = d.nseg;
                     n_comb = d.nb - c;
+                    // units: the segments, the dense ones several times
+                    std::vector<uint32_t> &base = q_dense[i];
+                    dense_units(d, hP, c, threads, (uint32_t)ctx->sm_count * 2, base);
+                    uint64_t extra = 0;
+                    for (size_t k = 0; k + 1 < base.size(); k++) {
+                        const uint64_t more = base[k + 1] - base[k] - 1, lo = (d.seg0 + k) * span, hi = lo + span;
+                        if (!more) continue;
+                        n_seg += more;
+                        uint64_t v = std::min<uint64_t>(d.r4, cpx_isqrt((u128)(hi - 1)));  // seg_levels
+                        if (lo) v = std::min<uint64_t>(v, cpx_isqrt((x - 1) / lo));
+                        const uint64_t nlv = host_pi(hP, v);
+                        if (nlv > c) extra += more * (nlv - c);
+                    }
+                    d.dense_segs = base.empty() ? 0 : (uint32_t)(base.size() - 1);
                     uint64_t ent = 0;
                     for (uint32_t b = c + 1; b <= d.nb; b++)
                         ent += segments_at_level(x, span, hP[b - 1], d.seg0, d.nseg);
                     q_ent[i] = ent;
+                    q_rows[i] = ent + extra;
                 }
             }
             p_ord[i + 1] = n_ord;
@@ -819,7 +921,7 @@ replan:  // again without the batch alpha when its shared sieve would not fit (b
     uint32_t lbits_max = 0;
     for (uint32_t i = 0; i < Q; i++) {
         if (!q_ent[i]) continue;
-        hard_entries += q_ent[i];
+        hard_entries += q_rows[i];
         hard_bytes += (double)q_ent[i] * (double)(1u << qd[i].lbits) / 8.0;
         lbits_max = std::max(lbits_max, qd[i].lbits);
     }
@@ -925,9 +1027,15 @@ replan:  // again without the batch alpha when its shared sieve would not fit (b
     const size_t qd_bytes = sizeof(QD) * Q, pre_bytes = (pre.size() * 8 + 15) & ~size_t(15);
     const size_t elv_bytes = elv.size() * sizeof(EasyLvl);
     const size_t grp_bytes = groups.size() * sizeof(HardGroup);
+    std::vector<uint32_t> dense;
+    for (uint32_t i = 0; i < (uint32_t)q_dense.size(); i++) {
+        qd[i].dense_off = (uint32_t)dense.size();
+        dense.insert(dense.end(), q_dense[i].begin(), q_dense[i].end());
+    }
+    const size_t dense_bytes = (dense.size() * 4 + 15) & ~size_t(15);
     const size_t pg_bytes = (units.size() * 8 + 15) & ~size_t(15), lo_bytes = (lvl_off.size() * 8 + 15) & ~size_t(15);
     const bool persist = shared && ctx->hard_persist;
-    const size_t stage_bytes = qd_bytes + pre_bytes + elv_bytes + grp_bytes + pg_bytes + lo_bytes;
+    const size_t stage_bytes = qd_bytes + pre_bytes + elv_bytes + grp_bytes + pg_bytes + lo_bytes + dense_bytes;
     const size_t acc_words = (size_t)Q * kAccStride;
     unsigned char *dbuf = (unsigned char *)ctx->b_work[0].get(stage_bytes + acc_words * 8 + 64);
     QD *d_qd = reinterpret_cast<QD *>(dbuf);
@@ -973,35 +1081,41 @@ replan:  // again without the batch alpha when its shared sieve would not fit (b
             pl.seg_off = ctx->b_work[3].as<uint64_t>(pl.n_seg + 1);
             pl.hard_cnt = ctx->b_work[4].as<uint32_t>(hard_entries + 1);
             pl.hard_ms = ctx->b_work[5].as<int32_t>(hard_entries + 1);
+            const size_t xb = wide ? 16 : 8;
+            unsigned char *lv = static_cast<unsigned char *>(ctx->b_lvpar.get((pl.n_comb + 1) * (xb + 8)));
+            pl.lvx = lv;
+            pl.lae = reinterpret_cast<uint2 *>(lv + (pl.n_comb + 1) * xb);
+            pl.dense = reinterpret_cast<const uint32_t *>(dbuf + stage_bytes - dense_bytes);
+        } else {
+            // snapshot pool for the heavy (sub-segment, level) leaf sets, counted on
+            // the host; the threshold doubles until the pool fits the budget
+            const size_t stride = hard_snapshot_stride(lbits_max - (uint32_t)(__builtin_ctz(threads) - 5));
+            const uint64_t budget = std::max<uint64_t>(1, ctx->hard_offload_bytes / (stride + sizeof(HardJob)));
+            uint64_t thr = offload0, njobs = 0;
+            while (thr) {
+                std::atomic<uint64_t> total(0);
+                parallel_blocks(nblk, [&](size_t k) {
+                    const size_t i1 = std::min<size_t>(Q, (k + 1) * kPlanBlock);
+                    for (size_t i = k * kPlanBlock; i < i1 && total.load() <= budget; i++) {
+                        const QD &d = qd[i];
+                        if (d.direct || d.nb <= c) continue;
+                        total += wide ? heavy_leaf_sets<u128>(d, hP, threads, thr, budget + 1)
+                                      : heavy_leaf_sets<uint64_t>(d, hP, threads, thr, budget + 1);
+                    }
+                });
+                njobs = total.load();
+                if (njobs <= budget) break;
+                thr = (thr >= (1ull << 40)) ? 0 : 2 * thr;
+            }
+            pl.offload_min = thr;
+            pl.max_jobs = thr ? (uint32_t)std::min<uint64_t>(njobs + 64, 0xFFFFFFF0ull) : 0;
+            pl.jobs = ctx->b_jobs.as<HardJob>(pl.max_jobs + 1);
+            uint64_t *ctl = ctx->b_jobctl.as<uint64_t>(pl.max_jobs + 4);
+            pl.njobs = reinterpret_cast<unsigned int *>(ctl);
+            pl.nsnap = reinterpret_cast<unsigned int *>(ctl + 1);
+            pl.job_units = ctl + 2;
+            pl.snap = static_cast<unsigned char *>(ctx->b_snap.get((pl.max_jobs + 1) * stride));
         }
-        // snapshot pool for the heavy (sub-segment, level) leaf sets, counted on
-        // the host; the threshold doubles until the pool fits the budget
-        const size_t stride = hard_snapshot_stride(lbits_max - (uint32_t)(__builtin_ctz(threads) - 5));
-        const uint64_t budget = std::max<uint64_t>(1, ctx->hard_offload_bytes / (stride + sizeof(HardJob)));
-        uint64_t thr = offload0, njobs = 0;
-        while (thr) {
-            std::atomic<uint64_t> total(0);
-            parallel_blocks(nblk, [&](size_t k) {
-                const size_t i1 = std::min<size_t>(Q, (k + 1) * kPlanBlock);
-                for (size_t i = k * kPlanBlock; i < i1 && total.load() <= budget; i++) {
-                    const QD &d = qd[i];
-                    if (d.direct || d.nb <= c) continue;
-                    total += wide ? heavy_leaf_sets<u128>(d, hP, threads, thr, budget + 1)
-                                  : heavy_leaf_sets<uint64_t>(d, hP, threads, thr, budget + 1);
-                }
-            });
-            njobs = total.load();
-            if (njobs <= budget) break;
-            thr = (thr >= (1ull << 40)) ? 0 : 2 * thr;
-        }
-        pl.offload_min = thr;
-        pl.max_jobs = thr ? (uint32_t)std::min<uint64_t>(njobs + 64, 0xFFFFFFF0ull) : 0;
-        pl.jobs = ctx->b_jobs.as<HardJob>(pl.max_jobs + 1);
-        uint64_t *ctl = ctx->b_jobctl.as<uint64_t>(pl.max_jobs + 4);
-        pl.njobs = reinterpret_cast<unsigned int *>(ctl);
-        pl.nsnap = reinterpret_cast<unsigned int *>(ctl + 1);
-        pl.job_units = ctl + 2;
-        pl.snap = static_cast<unsigned char *>(ctx->b_snap.get((pl.max_jobs + 1) * stride));
     }
     if (pl.n_easy) {
         // the chunk offsets, then (up to 1 GiB) the units' plans
@@ -1043,6 +1157,7 @@ replan:  // again without the batch alpha when its shared sieve would not fit (b
         memcpy(h_sh + grp_bytes, units.data(), units.size() * 8);
         memcpy(h_sh + grp_bytes + pg_bytes, lvl_off.data(), lvl_off.size() * 8);
     }
+    if (!dense.empty()) memcpy(stage.data() + stage_bytes - dense_bytes, dense.data(), dense.size() * 4);
     CPX_CUDA(cudaMemcpyAsync(dbuf, stage.data(), stage.size(), cudaMemcpyHostToDevice, ctx->stream));
     CPX_CUDA(cudaMemsetAsync(d_acc, 0, acc_words * 8 + 8, ctx->stream));  // and the unit counter
 

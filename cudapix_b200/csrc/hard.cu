@@ -7,37 +7,38 @@
 // contributes -mu(m) phi(u, b-1), which the sieve answers from the bitmap of
 // the segment holding u plus the survivors of level b-1 below it.
 //
-// One CTA owns one segment of 2^lbits odd numbers n = lo + 2i + 1; each of its
-// warps owns a contiguous sub-segment as a bitmap in shared memory with one
-// 8-bit survivor counter per 16-byte chunk (128 numbers), and walks the levels
-// b = c+1 .. B(seg) on its own, synchronising only inside the warp.  Per
-// level a warp (1) records its survivor count at level b-1, (2) if its
-// sub-segment holds leaves of p_b, scans the counters into lane prefixes and
-// answers each leaf as lane prefix + earlier counters of the owning lane +
-// popcounts in the chunk -- or, for a large candidate range, hands the level
-// to k_hard_leaves with a snapshot of the sub-segment, (3) crosses off p_b,
-// counting cleared bits and keeping the counters current.  The level
-// parameters (x/p, candidate range, first multiple) are computed 32 levels at
-// a time, one level per lane, and broadcast by shuffles.
+// One CTA owns one unit: a segment of 2^lbits odd numbers n = lo + 2i + 1 and
+// all of its leaves, or every nparts-th 32 table entries of their candidates
+// where the segment holds more leaves than the rest of its work (the early
+// segments: their number falls as 1/u^2).  Each warp owns a contiguous
+// sub-segment as a bitmap in shared memory with one 8-bit survivor counter per
+// 16-byte chunk (128 numbers), and walks the levels b = c+1 .. B(seg) on its
+// own, synchronising only inside the warp, 32 levels (a block) at a time: one
+// level per lane loads x/p, y/p and min(y, x/p^3) from a table filled once per
+// query and computes its candidate range and first multiple.
 //
-// Blocks of 32 levels whose primes have few multiples in a sub-segment (and no
-// leaf set for k_hard_leaves) go through at once instead: cross_levels takes
-// one multiple of each level a step, the block's candidates are walked as one
-// sequence, and each leaf is counted on the bitmap after the whole block plus
-// the bits up to u that its own and higher levels cleared, which cross_levels
-// notes down.  One level at a time such a level costs a warp some 250 issue
-// slots for a handful of multiples and one or two leaves, with most lanes
-// idle: integer issue bounds the kernel (81% of the slots), not memory.
-// On a B200: the sieve of pi(1e15) 2.82 -> 2.15 ms, of pi(1e17) 26.4 -> 20.1,
-// of pi(2e19) 1308 -> 904, of pi(1e12) 0.279 -> 0.184.
+// A block goes through at once when its primes have few multiples in the
+// sub-segment and its leaves are not many: cross_levels takes one multiple of
+// each level a step, the block's candidates are walked as one sequence, and
+// each leaf is counted on the bitmap after the whole block plus the bits up to
+// u that its own and higher levels cleared, which cross_levels notes down.
+// Else the levels go one by one: the warp (1) records its survivor count at
+// level b-1, (2) scans the counters into lane prefixes and answers each leaf
+// as lane prefix + earlier counters of the owning lane + popcounts in the
+// chunk, (3) crosses off p_b, counting cleared bits and keeping the counters
+// current.  After each block the CTA combines its warps: carries between
+// sub-segments enter the hard sum and the per-unit (count, Sum(-mu)) pairs go
+// to k_hard_combine, which adds the carries between segments.
 //
-// Every 32 levels the
-// CTA combines its warps: carries between sub-segments enter the hard sum and
-// the per-segment (count, Sum(-mu)) pairs go to k_hard_combine, which adds the
-// carries between segments.
+// Integer issue and the latency of a warp's chain of levels bound the kernel,
+// not memory.  Hard leaves on a B200, one level at a time with the heavy leaf
+// sets in a kernel of their own, then blocks at once, then units split by
+// their leaves and leaves found for a run of levels before they are needed:
+// pi(1e12) 0.300, 0.202, 0.205 ms; pi(1e15) 3.05, 2.43, 1.93; pi(1e17) 36.3,
+// 30.2, 22.3; pi(1.9e19) 1370, 950, 628.
 //
 // This is the sieve of lone queries and small batches.  Larger batches share
-// the sieve between queries (hard_shared.cu); k_hard_leaves serves both.
+// the sieve between queries (hard_shared.cu).
 #include <algorithm>
 #include <mutex>
 
@@ -45,13 +46,52 @@
 
 namespace cpx {
 
-// A block of 32 levels is crossed off at once (cross_levels) when its smallest
-// prime has at most this many multiples in a warp's sub-segment.  Below that
-// the bits a block clears outnumber the leaves it answers, and each leaf is
-// compared with all of them.  On a B200 the sieve of pi(1e15) took 2.82 ms one
-// level at a time and 2.52 / 2.15 / 2.59 with 8 / 16 / 32 here; of pi(2e19)
-// 1308 and 929 / 904 / 888.
-constexpr uint32_t kLevelWindows = 16;
+// The unit `u` of a query's units (relative to its first): its segment
+// (relative to seg0), which part of the segment's leaves it takes, of how many.
+struct UnitSeg {
+    uint64_t seg;
+    uint32_t part, nparts;
+};
+__device__ __forceinline__ UnitSeg unit_seg(const QD &d, const uint32_t *__restrict__ dense, uint64_t u)
+{
+    const uint32_t K = d.dense_segs;
+    if (!K) return {u, 0u, 1u};
+    const uint32_t *base = dense + d.dense_off;
+    const uint32_t nu = __ldg(base + K);
+    if (u >= nu) return {K + (u - nu), 0u, 1u};
+    uint32_t lo = 0, hi = K;  // base[lo] <= u < base[hi]
+    while (hi - lo > 1) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (__ldg(base + mid) <= u) lo = mid;
+        else hi = mid;
+    }
+    const uint32_t b0 = __ldg(base + lo);
+    return {lo, (uint32_t)u - b0, __ldg(base + lo + 1) - b0};
+}
+// the first unit of a query's segment `seg` (relative to seg0)
+__device__ __forceinline__ uint64_t seg_unit(const QD &d, const uint32_t *__restrict__ dense, uint64_t seg)
+{
+    const uint32_t K = d.dense_segs;
+    if (!K) return seg;
+    const uint32_t *base = dense + d.dense_off;
+    return seg < K ? __ldg(base + seg) : __ldg(base + K) + (seg - K);
+}
+
+template <class XT> __device__ __forceinline__ XT shfl_xt(XT v, uint32_t src)
+{
+    if (sizeof(XT) == 8) return (XT)__shfl_sync(FULL, (unsigned long long)v, src);
+    const unsigned long long a0 = __shfl_sync(FULL, (unsigned long long)v, src);
+    const unsigned long long a1 = __shfl_sync(FULL, (unsigned long long)((u128)v >> 64), src);
+    return (XT)(((u128)a1 << 64) | a0);
+}
+
+// A block of levels goes through at once when its smallest prime has at most
+// kLevelWindows multiples in a warp's sub-segment, and when its leaves times
+// the bits it clears (each leaf is compared with all of them) stay below
+// kLevelLeafEvents a level: one by one, a level costs about 250 issue slots
+// whatever its leaves, which 2048 comparisons of a warp's lanes take too.
+constexpr uint32_t kLevelWindows = 64;
+constexpr uint32_t kLevelLeafEvents = 2048;
 
 template <class XT>
 __global__ void __launch_bounds__(512, 2) k_hard(const QD *__restrict__ qd, uint32_t Q,
@@ -60,12 +100,11 @@ __global__ void __launch_bounds__(512, 2) k_hard(const QD *__restrict__ qd, uint
                                               const uint64_t *__restrict__ seg_off,
                                               const uint32_t *__restrict__ P, const int32_t *__restrict__ MU,
                                               const cpx_pient *__restrict__ Tpi,
+                                              const uint64_t *__restrict__ pre_comb, const XT *__restrict__ lvx,
+                                              const uint2 *__restrict__ lae, const uint32_t *__restrict__ dense,
                                               uint32_t *__restrict__ out_cnt, int32_t *__restrict__ out_ms,
                                               uint64_t cap, unsigned long long *__restrict__ acc,
-                                              uint32_t lbits_max, HardJob *__restrict__ jobs,
-                                              unsigned int *__restrict__ njobs, uint64_t *__restrict__ job_units,
-                                              unsigned char *__restrict__ snap, uint32_t max_jobs,
-                                              uint32_t lbits_sub_max, uint32_t offload_min)
+                                              uint32_t lbits_max)
 {
     extern __shared__ uint4 smem4[];
     const uint64_t unit = blockIdx.x;
@@ -81,14 +120,15 @@ __global__ void __launch_bounds__(512, 2) k_hard(const QD *__restrict__ qd, uint
     const uint32_t CPT = NC / T;   // chunks per lane (>= 1)
     const int s = __ffs(CPT) - 1;  // log2 CPT
     const uint32_t Lw = L / NW;    // bits of a warp's sub-segment
-    const uint64_t seg = unit - pre_seg[q] + d.seg0;
-    const uint64_t lo = seg * 2 * (uint64_t)L;
+    const UnitSeg us = unit_seg(d, dense, unit - pre_seg[q]);
+    const uint64_t lo = (us.seg + d.seg0) * 2 * (uint64_t)L;
     const uint64_t lo_w = lo + 2 * (uint64_t)Lw * warp, hi_w = lo_w + 2 * (uint64_t)Lw;
     const bool q41 = hi_w <= (1ull << 41);  // leaf quotients lie in [lo_w, hi_w)
     const uint64_t off = seg_off[unit];
     if (off + (B - c) > cap) return;  // the host sized the ragged outputs exactly; never write past them
-    const XT x = xload<XT>(d);
     const uint64_t y = d.y;
+    const uint64_t lv0 = pre_comb[q];  // the query's rows of the level table
+    const uint32_t step = 32 * us.nparts, first = 32 * us.part;  // this unit's candidate entries
 
     // carve the shared block (sized for lbits_max)
     unsigned char *sp = reinterpret_cast<unsigned char *>(smem4);
@@ -104,9 +144,12 @@ __global__ void __launch_bounds__(512, 2) k_hard(const QD *__restrict__ qd, uint
     o = (o + 15) & ~size_t(15);
     i128 *s_red = reinterpret_cast<i128 *>(sp + o);
     o += 32 * sizeof(i128);
-    uint32_t *lbuf = reinterpret_cast<uint32_t *>(sp + o) + kLeafBuf * warp;  // this warp's gathered leaves
-    o += NW * kLeafBuf * 4;
-    uint32_t *ev = reinterpret_cast<uint32_t *>(sp + o) + kEvCap * warp;      // this warp's cleared bits
+    uint2 *lbuf = reinterpret_cast<uint2 *>(sp + o) + kLeafCap * warp;        // this warp's gathered leaves
+    o += NW * kLeafCap * sizeof(uint2);
+    // this warp's cleared bits (levels at once) or the prefixes of its chunks
+    // within their lanes (levels one by one)
+    uint32_t *ev = reinterpret_cast<uint32_t *>(sp + o + ev_bytes(d.lbits, T) * warp);
+    uint16_t *pre16 = reinterpret_cast<uint16_t *>(ev) - CPT * 32 * warp;  // by the segment's chunk
     uint32_t *wl = loff + 32 * warp;  // this warp's lane prefixes
 
     const uint32_t c0 = CPT * tid;  // first owned chunk (of the segment)
@@ -116,54 +159,96 @@ __global__ void __launch_bounds__(512, 2) k_hard(const QD *__restrict__ qd, uint
     uint32_t tot = __reduce_add_sync(FULL, cnt0);  // survivors of this warp's sub-segment
     __syncwarp();
 
-    const BoundDiv bd_lo = bound_div(lo_w), bd_hi = bound_div(hi_w);
-    auto sub_count = [&](uint64_t uu) -> uint32_t { return sub_survivors(uu, lo_w, wl, cnt8, bm, CPT, s, warp); };
+    const Recip r_lo{lo_w, lo_w ? 1.0 / (double)lo_w : 0.0}, r_hi{hi_w, 1.0 / (double)hi_w};
 
     int64_t S = 0;       // this lane's share of the hard sum (survivor counts within sub-segments)
     i128 Sx = 0;         // warp 0: carries between the CTA's sub-segments
     uint32_t grp = 0;
     for (uint32_t gb = c + 1; gb <= B; gb += 32, grp++) {
         const uint32_t nl = min(32u, B - gb + 1);
-        // ---- level parameters, one level per lane
-        LvlPar<XT> lv;
-        lv.p = 0;
-        lv.mlo = lv.mhi = lv.r0 = 0;
-        lv.i0 = 0xFFFFFFFFu;
-        lv.xp = 0;
-        if (lane < nl) level_params<XT>(lv, x, y, P[gb + lane - 1], lo_w, hi_w, bd_lo, bd_hi);
-        const uint32_t lp = lv.p, lmlo = lv.mlo, lmhi = lv.mhi, lr0 = lv.r0, li0 = lv.i0;
-        const XT lxp = lv.xp;
-        // levels of the block with candidates in the sub-segment (most levels of
-        // the high segments have none: they only cross off)
-        const unsigned act = __ballot_sync(FULL, lane < nl && lv.mhi > lv.mlo);
-        LvlSum mine = {0, 0, 0xFFFFFFFFu};
-        LvlSum *ar = area + (grp & 1) * NW * 32;
-        // table entries of each level's candidates: pi-table words of the
-        // prime-only levels, 4-m groups of packed mu*lpf of the others
+        // ---- level parameters, one level per lane: p, x/p, the candidates
+        // (mlo, mhi] with u = xp/m in the sub-segment, the first multiple
+        uint32_t lp = 0, lmlo = 0, lmhi = 0, lr0 = 0, li0 = 0xFFFFFFFFu;
+        XT lxp = 0;
+        if (lane < nl) {
+            const uint64_t li = lv0 + (gb - c - 1) + lane;
+            lp = P[gb + lane - 1];
+            lxp = lvx[li];
+            const uint2 ae = lae[li];
+            uint64_t a = ae.x, e = ae.y;
+            const XT t1 = div_recip(lxp, r_hi);
+            if (t1 > (XT)a) a = (uint64_t)t1;
+            if (lo_w) {
+                const XT t2 = div_recip(lxp, r_lo);
+                if (t2 < (XT)e) e = (uint64_t)t2;
+            }
+            lmlo = (uint32_t)a;
+            lmhi = (uint32_t)(e > a ? e : a);
+            cross_params(lp, lo_w, hi_w, lr0, li0);
+        }
+        // Items of each level's candidates: the primes P[k] of a prime-only level
+        // (m = q > max(mlo, p)), each a leaf, or the 4-m groups of packed mu*lpf.
+        // p^2 > y from some level on, so the group levels of a block come first.
         const bool prime_j = (uint64_t)lp * lp > y;
         const uint32_t qa_j = lmlo > lp ? lmlo : lp;
-        uint32_t nw_j = 0, ng_j = 0;
-        if (lane < nl && lmhi > lmlo) {
-            if (!prime_j) ng_j = ((lmhi - 1) >> 3) - ((lmlo + 1) >> 3) + 1;
-            else if (lmhi > qa_j) nw_j = ((lmhi - 1) >> 7) - (qa_j >> 7) + 1;
+        uint32_t nw_j = 0, ng_j = 0, k0_j = 0;
+        if (lmhi > lmlo) {
+            if (!prime_j) {
+                ng_j = ((lmhi - 1) >> 3) - ((lmlo + 1) >> 3) + 1;
+            } else if (lmhi > qa_j) {
+                k0_j = (uint32_t)cpx_pi_ge2(Tpi, qa_j);
+                nw_j = (uint32_t)cpx_pi_ge2(Tpi, lmhi) - k0_j;
+            }
         }
-        const bool heavy_j = max_jobs && offload_min && 8 * nw_j + 4 * ng_j >= offload_min;
+        LvlSum *ar = area + (grp & 1) * NW * 32;
+        ar[warp * 32 + lane].ms = 0;
+        // the levels' leaves at most, and about one bit in seven of a level's
+        // multiples is still set
+        const uint32_t lf_j = min(nw_j, 1u << 20) + 4 * min(ng_j, 1u << 20);
         const uint32_t pmin = __shfl_sync(FULL, lp, 0);
-        if ((uint64_t)pmin * kLevelWindows >= Lw && !__any_sync(FULL, heavy_j)) {
-            // ---- the block's levels at once
-            const bool leaves = __any_sync(FULL, (nw_j | ng_j) != 0);
+        bool at_once = (uint64_t)pmin * kLevelWindows >= Lw;
+        if (at_once) {
+            const uint32_t est = __reduce_add_sync(FULL, min(nw_j + ng_j, 1u << 26)) / us.nparts;
+            at_once = (uint64_t)est * (nl * (Lw / pmin + 1) / 7 + 4) <= (uint64_t)nl * kLevelLeafEvents;
+        }
+        uint32_t mine_cnt = 0;
+        // item offsets of the levels (32 bits: a level of 2^26 items or more only goes alone)
+        uint32_t ex_w, ex_g;
+        const uint32_t tot_w = warp_place(min(nw_j, 1u << 26), lane, ex_w),
+                       tot_g = warp_place(min(ng_j, 1u << 26), lane, ex_g);
+
+        // item f of the block's primes: its level (the lane holding it) and prime
+        auto prime_item = [&](uint32_t f, uint32_t end, uint32_t &jq) -> uint32_t {
+            jq = item_owner(ex_w, f);
+            const uint32_t k = __shfl_sync(FULL, k0_j - ex_w, jq) + f;
+            return f < end ? __ldg(P + k) : 1u;
+        };
+        // item f of the block's groups: its level, first m index / 4, valid m's and their signs
+        auto group_item = [&](uint32_t f, uint32_t end, uint32_t &jq, uint64_t &g4, uint32_t &neg) -> uint32_t {
+            jq = item_owner(ex_g, f);
+            const uint32_t exq = __shfl_sync(FULL, ex_g, jq), pq = __shfl_sync(FULL, lp, jq);
+            const uint64_t mlq = __shfl_sync(FULL, lmlo, jq), mhq = __shfl_sync(FULL, lmhi, jq);
+            const uint64_t i_lo = (mlq + 1) >> 1, i_hi = (mhq - 1) >> 1;
+            neg = 0;
+            g4 = (i_lo >> 2) + (f - exq);
+            return f < end ? valid_group(__ldg(reinterpret_cast<const int4 *>(MU) + g4), g4, i_lo, i_hi, pq, &neg) : 0u;
+        };
+        // bits [0, kk) of the sub-segment are the numbers up to u = xp / m
+        auto leaf_bits = [&](XT xp, double xpd, uint32_t m) -> uint32_t {
+            return ((uint32_t)leaf_quot(xp, xpd, m, q41) - (uint32_t)lo_w + 1u) >> 1;
+        };
+
+        if (at_once) {
             uint32_t i = li0, w_end = pmin, cleared = 0;
-            ar[warp * 32 + lane].ms = 0;
-            if (!leaves) {
+            if (!(tot_w | tot_g)) {
                 cross_levels<false>(bm, cnt8, lp, i, pmin, w_end, cleared, s, CPT * 32 * warp, lane, Lw, ev, 0);
             } else {
-                uint2 *lb2 = reinterpret_cast<uint2 *>(lbuf);
-                constexpr uint32_t kCap2 = kLeafBuf / 2;
-                uint32_t ex_w, ex_g;
-                const uint32_t tot_w = warp_place(nw_j, lane, ex_w), tot_g = warp_place(ng_j, lane, ex_g);
-                uint32_t k_lo = 0;  // the slice's leaves have their counts' bits [0, kk), k_lo < kk <= k_hi
+                // Slices of the sub-segment, as many as the bits cleared in it fill
+                // the event buffer (nearly always one): a slice's leaves have k_lo <
+                // kk <= k_hi.
+                uint32_t k_lo = 0;
                 for (;;) {
-                    // cleared bits of the earlier slices at this lane's level and above
+                    // bits of the earlier slices cleared by this lane's level and above
                     uint32_t suf = cleared;
 #pragma unroll
                     for (int oo = 1; oo < 32; oo <<= 1) {
@@ -173,271 +258,214 @@ __global__ void __launch_bounds__(512, 2) k_hard(const QD *__restrict__ qd, uint
                     const uint32_t nev = cross_levels<true>(bm, cnt8, lp, i, pmin, w_end, cleared, s, CPT * 32 * warp,
                                                             lane, Lw, ev, kEvCap);
                     const uint32_t k_hi = min(w_end - pmin, Lw);
-                    if (lane < 4 && nev + lane < kEvCap) ev[nev + lane] = kEvMask;  // the last four events
-                    // lane prefixes of the sub-segment from the chunk counters
+                    if (lane < 4 && nev + lane < kEvCap) ev[nev + lane] = kEvMask;  // fills the last four
                     uint32_t off0;
                     warp_place(counter_sum(cnt8 + c0, CPT), lane, off0);
                     wl[lane] = off0;
-                    uint32_t nbuf = 0;
-                    // Answers the gathered leaves (m, level k | (mu(m) = -1) << 31): the
-                    // survivors of level b - 1 up to u are those after the whole block
-                    // and the bits up to u that levels b and above took.
-                    auto flush = [&] {
-                        __syncwarp();
-                        for (uint32_t j0 = 0; j0 < nbuf; j0 += 32) {
-                            const bool on = j0 + lane < nbuf;
-                            uint2 e = make_uint2(1, 0);
-                            if (on) e = lb2[j0 + lane];
-                            const uint32_t key = e.y & 31u;
-                            XT xk;
-                            if (sizeof(XT) == 8) {
-                                xk = (XT)__shfl_sync(FULL, (unsigned long long)lxp, key);
-                            } else {
-                                const unsigned long long a0 = __shfl_sync(FULL, (unsigned long long)lxp, key);
-                                const unsigned long long a1 =
-                                    __shfl_sync(FULL, (unsigned long long)((u128)lxp >> 64), key);
-                                xk = (XT)(((u128)a1 << 64) | a0);
-                            }
-                            uint32_t cv = __shfl_sync(FULL, suf, key);
-                            if (on) {
-                                const uint64_t uu = leaf_quot(xk, (double)(uint64_t)xk, e.x, q41);
-                                const uint32_t kk = ((uint32_t)uu - (uint32_t)lo_w + 1u) >> 1;
-                                if (kk <= k_hi && (kk > k_lo || !k_lo)) {
-                                    cv += sub_count(uu);
-                                    const uint32_t kmin = key << kEvBit;
-                                    for (uint32_t t = 0; t < nev; t += 4) {
-                                        const uint4 v = *reinterpret_cast<const uint4 *>(ev + t);
-                                        cv += (v.x >= kmin && (v.x & kEvMask) < kk) + (v.y >= kmin && (v.y & kEvMask) < kk) +
-                                              (v.z >= kmin && (v.z & kEvMask) < kk) + (v.w >= kmin && (v.w & kEvMask) < kk);
-                                    }
-                                    const bool plus = (e.y >> 31) != 0;
-                                    if (plus) S += cv;
-                                    else S -= cv;
-                                    atomicAdd(&ar[warp * 32 + key].ms, plus ? 1 : -1);
-                                }
-                            }
+                    __syncwarp();
+                    // One leaf a lane: the survivors of level b - 1 up to u are those
+                    // after the whole block and the bits up to u that levels b and
+                    // above took.
+                    auto answer = [&](bool on, uint32_t m, uint32_t key, bool plus) {
+                        const XT xk = shfl_xt(lxp, key);
+                        uint32_t cv = __shfl_sync(FULL, suf, key);
+                        if (!on) return;
+                        const uint32_t kk = leaf_bits(xk, (double)(uint64_t)xk, m);
+                        if (kk > k_hi || (kk <= k_lo && k_lo)) return;
+                        cv += sub_survivors_bits(kk, wl, cnt8, bm, CPT, s, warp);
+                        const uint32_t kmin = key << kEvBit;
+                        for (uint32_t t = 0; t < nev; t += 4) {
+                            const uint4 v = *reinterpret_cast<const uint4 *>(ev + t);
+                            cv += (v.x >= kmin && (v.x & kEvMask) < kk) + (v.y >= kmin && (v.y & kEvMask) < kk) +
+                                  (v.z >= kmin && (v.z & kEvMask) < kk) + (v.w >= kmin && (v.w & kEvMask) < kk);
                         }
-                        __syncwarp();
-                        nbuf = 0;
+                        if (plus) S += cv;
+                        else S -= cv;
+                        atomicAdd(&ar[warp * 32 + key].ms, plus ? 1 : -1);
                     };
-                    for (uint32_t base = 0; base < tot_w; base += 32) {
-                        const uint32_t f = base + lane;
-                        const uint32_t jq = item_owner(ex_w, f);
-                        const uint32_t exq = __shfl_sync(FULL, ex_w, jq);
-                        const uint32_t qaq = __shfl_sync(FULL, qa_j, jq), mhq = __shfl_sync(FULL, lmhi, jq);
-                        uint64_t qb = 0, wq = 0;
-                        if (f < tot_w) {
-                            wq = (qaq >> 7) + (f - exq);
-                            qb = __ldg(reinterpret_cast<const ulonglong2 *>(Tpi) + wq).x & range_mask(wq, qaq, mhq);
-                        }
-                        // dense rounds (over 128 leaves) go in halves and quarters of a word
-                        for (uint32_t part = 0; __any_sync(FULL, qb != 0); part++) {
-                            uint64_t now = qb;
-                            if (__reduce_add_sync(FULL, (uint32_t)__popcll(qb)) > kCap2) now = qb & (0xFull << (4 * part));
-                            qb &= ~now;
-                            uint32_t off;
-                            const uint32_t tot_r = warp_place((uint32_t)__popcll(now), lane, off);
-                            if (nbuf + tot_r > kCap2) flush();
-                            uint32_t kk = nbuf + off;
-                            while (now) {
-                                const int j = __ffsll((long long)now) - 1;
-                                now &= now - 1;
-                                lb2[kk++] = make_uint2((uint32_t)(128 * wq + 2 * j + 1), jq | 0x80000000u);
+                    for (uint32_t base = first; base < tot_w; base += step) {
+                        uint32_t jq;
+                        const uint32_t m = prime_item(base + lane, tot_w, jq);
+                        answer(base + lane < tot_w, m, jq, true);  // mu(q) = -1
+                    }
+                    if (tot_g) {
+                        uint32_t nbuf = 0;
+                        auto flush = [&] {
+                            __syncwarp();
+                            for (uint32_t j0 = 0; j0 < nbuf; j0 += 32) {
+                                const bool on = j0 + lane < nbuf;
+                                const uint2 e = on ? lbuf[j0 + lane] : make_uint2(1, 0);
+                                answer(on, e.x, e.y & 31u, (e.y >> 31) != 0);
+                            }
+                            __syncwarp();
+                            nbuf = 0;
+                        };
+                        for (uint32_t base = first; base < tot_g; base += step) {
+                            uint32_t jq, neg, off_l;
+                            uint64_t g4;
+                            uint32_t vm = group_item(base + lane, tot_g, jq, g4, neg);
+                            const uint32_t tot_r = warp_place((uint32_t)__popc(vm), lane, off_l);
+                            if (nbuf + tot_r > kLeafCap) flush();
+                            for (uint32_t kk = nbuf + off_l; vm; kk++) {
+                                const int kq = __ffs(vm) - 1;
+                                vm &= vm - 1;
+                                lbuf[kk] = make_uint2((uint32_t)(2 * (4 * g4 + kq) + 1), jq | (((neg >> kq) & 1u) << 31));
                             }
                             nbuf += tot_r;
                         }
+                        flush();
                     }
-                    for (uint32_t base = 0; base < tot_g; base += 32) {
-                        const uint32_t f = base + lane;
-                        const uint32_t jq = item_owner(ex_g, f);
-                        const uint32_t exq = __shfl_sync(FULL, ex_g, jq), pq = __shfl_sync(FULL, lp, jq);
-                        const uint64_t mlq = __shfl_sync(FULL, lmlo, jq), mhq = __shfl_sync(FULL, lmhi, jq);
-                        const uint64_t i_lo = (mlq + 1) >> 1, i_hi = (mhq - 1) >> 1;
-                        uint32_t neg = 0, vm = 0;
-                        uint64_t g4 = 0;
-                        if (f < tot_g) {
-                            g4 = (i_lo >> 2) + (f - exq);
-                            vm = valid_group(__ldg(reinterpret_cast<const int4 *>(MU) + g4), g4, i_lo, i_hi, pq, &neg);
-                        }
-                        uint32_t off;
-                        const uint32_t tot_r = warp_place((uint32_t)__popc(vm), lane, off);
-                        if (nbuf + tot_r > kCap2) flush();
-                        uint32_t kk = nbuf + off;
-                        while (vm) {
-                            const int kq = __ffs(vm) - 1;
-                            vm &= vm - 1;
-                            lb2[kk++] = make_uint2((uint32_t)(2 * (4 * g4 + kq) + 1), jq | (((neg >> kq) & 1u) << 31));
-                        }
-                        nbuf += tot_r;
-                    }
-                    flush();
                     if (k_hi == Lw) break;
                     k_lo = k_hi;
+                    __syncwarp();
                 }
             }
             uint32_t before;
             const uint32_t all = warp_place(cleared, lane, before);
-            mine.cnt = tot - before;
+            mine_cnt = tot - before;
             tot -= all;
-            mine.ms = ar[warp * 32 + lane].ms;
-        } else
-        for (uint32_t k = 0; k < nl; k++) {
-            const uint32_t b = gb + k;
-            const uint32_t p = __shfl_sync(FULL, lp, k);
-            const uint32_t cnt_b = tot;
-            int32_t ms_b = 0;
-            uint32_t job_b = 0xFFFFFFFFu;
-            if ((act >> k) & 1u) {
-                const uint32_t mlo = __shfl_sync(FULL, lmlo, k), mhi = __shfl_sync(FULL, lmhi, k);
-                XT xp;
-                if (sizeof(XT) == 8) {
-                    xp = (XT)__shfl_sync(FULL, (unsigned long long)lxp, k);
-                } else {
-                    const unsigned long long a0 = __shfl_sync(FULL, (unsigned long long)lxp, k);
-                    const unsigned long long a1 = __shfl_sync(FULL, (unsigned long long)((u128)lxp >> 64), k);
-                    xp = (XT)(((u128)a1 << 64) | a0);
-                }
-                // lane prefixes of the sub-segment from the chunk counters
-                const uint32_t run = counter_sum(cnt8 + c0, CPT);
-                uint32_t inc = run;
-#pragma unroll
-                for (int oo = 1; oo < 32; oo <<= 1) {
-                    const uint32_t t = __shfl_up_sync(FULL, inc, oo);
-                    if (lane >= (uint32_t)oo) inc += t;
-                }
-                wl[lane] = inc - run;
-                __syncwarp();
-                const bool prime_lvl = (uint64_t)p * p > y;
-                const uint64_t qa = mlo > p ? mlo : p;
-                uint64_t work;
-                if (prime_lvl) work = (mhi > qa) ? 8 * ((((uint64_t)mhi - 1) >> 7) - (qa >> 7) + 1) : 0;
-                else work = ((((uint64_t)mhi - 1) >> 1) - (((uint64_t)mlo + 1) >> 1) + 1);
-                bool offloaded = false;
-                if (max_jobs && offload_min && work >= offload_min) {
-                    unsigned int j = 0;
-                    if (lane == 0) j = atomicAdd(njobs, 1u);
-                    j = __shfl_sync(FULL, j, 0);
-                    if (j < max_jobs) {
-                        offloaded = true;
-                        job_b = j;
-                        const size_t stride = snap_stride(lbits_sub_max);
-                        uint4 *sb = reinterpret_cast<uint4 *>(snap + (size_t)j * stride);
-                        uint32_t *spre = reinterpret_cast<uint32_t *>(sb + ((size_t(1) << lbits_sub_max) >> 7));
-                        snapshot_chunks(sb, spre, bm, cnt8, cw0, c0, CPT, s, wl[lane]);
-                        if (lane == 0) {
-                            HardJob J;
-                            J.q = q;
-                            J.b = b;
-                            J.p = p;
-                            J.kind = prime_lvl ? 1u : 0u;
-                            J.mlo = prime_lvl ? qa : mlo;
-                            J.mhi = mhi;
-                            J.lo = lo_w;
-                            J.slot = off + (b - c - 1);
-                            J.nunits = prime_lvl ? (work / 8 + kJobWords - 1) / kJobWords
-                                                 : (((((uint64_t)mhi - 1) >> 1) >> 2) -
-                                                    ((((uint64_t)mlo + 1) >> 1) >> 2) + kJobGroups) /
-                                                       kJobGroups;
-                            J.carry = 0;  // filled in by the group combine below
-                            J.snap = j;
-                            job_units[j] = J.nunits;
-                            J.xp = (u128)xp;
-                            jobs[j] = J;
-                        }
-                    }
-                }
-                if (!offloaded) {
-                    // The lanes gather the level's leaves (m, with bit 31 set when
-                    // mu(m) = -1) into the warp's buffer and answer them 32 at a time,
-                    // so that a lane with many candidates does not hold up the others.
-                    int32_t msl = 0;
-                    uint32_t nbuf = 0;
-                    const double xpd = (double)(uint64_t)xp;
-                    auto flush = [&] {
-                        __syncwarp();
-                        for (uint32_t jj = lane; jj < nbuf; jj += 32) {
-                            const uint32_t e = lbuf[jj];
-                            const uint32_t cv = sub_count(leaf_quot(xp, xpd, e & 0x7FFFFFFFu, q41));
-                            if (e >> 31) {
-                                S += cv;
-                                msl += 1;
-                            } else {
-                                S -= cv;
-                                msl -= 1;
-                            }
-                        }
-                        __syncwarp();
-                        nbuf = 0;
-                    };
-                    auto place = [&](uint32_t n, uint32_t &off) -> uint32_t { return warp_place(n, lane, off); };
-                    if (prime_lvl) {
-                        // m must be a prime q > p: walk the pi-table bitmap of (max(mlo, p), mhi]
-                        if (mhi > qa) {
-                            const uint64_t w0q = qa >> 7, w1q = ((uint64_t)mhi - 1) >> 7;
-                            for (uint64_t wb = w0q; wb <= w1q; wb += 32) {
-                                const uint64_t wq = wb + lane;
-                                uint64_t qb = 0;
-                                if (wq <= w1q)
-                                    qb = __ldg(reinterpret_cast<const ulonglong2 *>(Tpi) + wq).x & range_mask(wq, qa, mhi);
-                                uint32_t off;
-                                const uint32_t tot_r = place((uint32_t)__popcll(qb), off);
-                                if (tot_r > kLeafBuf) {  // a dense round: each lane answers its own word
-                                    while (qb) {
-                                        const int j = __ffsll((long long)qb) - 1;
-                                        qb &= qb - 1;
-                                        S += sub_count(leaf_quot(xp, xpd, 128 * wq + 2 * j + 1, q41));  // mu(q) = -1
-                                        msl += 1;
-                                    }
-                                    continue;
-                                }
-                                if (nbuf + tot_r > kLeafBuf) flush();
-                                uint32_t kk = nbuf + off;
-                                while (qb) {
-                                    const int j = __ffsll((long long)qb) - 1;
-                                    qb &= qb - 1;
-                                    lbuf[kk++] = (uint32_t)(128 * wq + 2 * j + 1) | 0x80000000u;
-                                }
-                                nbuf += tot_r;
-                            }
-                        }
+        } else {
+            // Runs of levels [ka, kb) whose leaves fit the warp's buffer: all of
+            // them are found first (level by level in order: kk | (mu(m) = -1) << 31
+            // and the level), then each level answers its own.  A level with more
+            // leaves, or one split over units, answers them as it finds them.
+            uint32_t ex_l;
+            warp_place(lf_j, lane, ex_l);
+            uint32_t kb = 0;   // levels found
+            uint32_t st = 0, en = 0;  // this lane's level: its leaves in the buffer
+            bool dense = false;
+            for (uint32_t k = 0; k < nl; k++) {
+                if (k == kb) {
+                    const uint32_t e0 = __shfl_sync(FULL, ex_l, k);
+                    const unsigned fit = __ballot_sync(FULL, lane < k || ex_l + lf_j - e0 <= kLeafCap);
+                    kb = min(fit == FULL ? 32u : (uint32_t)__ffs(~fit) - 1, nl);
+                    dense = us.nparts > 1 || kb == k;
+                    if (dense) {
+                        kb = k + 1;
                     } else {
-                        // any squarefree m with lpf(m) > p: 16-byte loads of packed mu*lpf
-                        const uint64_t i_lo = ((uint64_t)mlo + 1) >> 1, i_hi = ((uint64_t)mhi - 1) >> 1;
-                        for (uint64_t gb = i_lo >> 2; gb <= (i_hi >> 2); gb += 32) {
-                            const uint64_t g = gb + lane;
-                            uint32_t neg = 0, vm = 0;
-                            if (g <= (i_hi >> 2))
-                                vm = valid_group(__ldg(reinterpret_cast<const int4 *>(MU) + g), g, i_lo, i_hi, p, &neg);
-                            uint32_t off;
-                            const uint32_t tot_r = place((uint32_t)__popc(vm), off);
-                            if (nbuf + tot_r > kLeafBuf) flush();
-                            uint32_t kk = nbuf + off;
-                            while (vm) {
+                        uint32_t nbuf = 0;
+                        const uint32_t gs = __shfl_sync(FULL, ex_g, k), ws = __shfl_sync(FULL, ex_w, k);
+                        const uint32_t ge = __shfl_sync(FULL, ex_g + ng_j, kb - 1),
+                                       we = __shfl_sync(FULL, ex_w + nw_j, kb - 1);
+                        for (uint32_t base = gs; base < ge; base += 32) {
+                            uint32_t jq, neg, off_l;
+                            uint64_t g4;
+                            uint32_t vm = group_item(base + lane, ge, jq, g4, neg);
+                            const XT xk = shfl_xt(lxp, jq);
+                            const double xkd = (double)(uint64_t)xk;
+                            const uint32_t tot_r = warp_place((uint32_t)__popc(vm), lane, off_l);
+                            for (uint32_t t = nbuf + off_l; vm; t++) {
                                 const int kq = __ffs(vm) - 1;
                                 vm &= vm - 1;
-                                lbuf[kk++] = (uint32_t)(2 * (4 * g + kq) + 1) | (((neg >> kq) & 1u) << 31);
+                                lbuf[t] = make_uint2(leaf_bits(xk, xkd, (uint32_t)(2 * (4 * g4 + kq) + 1)) |
+                                                         (((neg >> kq) & 1u) << 31),
+                                                     jq);
                             }
                             nbuf += tot_r;
                         }
+                        for (uint32_t base = ws; base < we; base += 32) {
+                            uint32_t jq;
+                            const uint32_t m = prime_item(base + lane, we, jq);
+                            const XT xk = shfl_xt(lxp, jq);
+                            if (base + lane < we)
+                                lbuf[nbuf + base + lane - ws] =
+                                    make_uint2(leaf_bits(xk, (double)(uint64_t)xk, m) | 0x80000000u, jq);
+                        }
+                        nbuf += we - ws;
+                        __syncwarp();
+                        // the first buffer entry of this lane's level, and of the next
+                        st = 0;
+                        for (uint32_t half = kLeafCap / 2; half; half >>= 1)
+                            if (st + half <= nbuf && lbuf[st + half - 1].y < lane) st += half;
+                        if (st < nbuf && lbuf[st].y < lane) st++;
+                        en = __shfl_down_sync(FULL, st, 1);
+                        if (lane == 31) en = nbuf;
                     }
-                    flush();
-                    ms_b = __reduce_add_sync(FULL, msl);
                 }
+                const uint32_t p = __shfl_sync(FULL, lp, k);
+                if (lane == k) mine_cnt = tot;
+                const uint32_t nw = __shfl_sync(FULL, nw_j, k), ng = __shfl_sync(FULL, ng_j, k);
+                const uint32_t lb = __shfl_sync(FULL, st, k), le = __shfl_sync(FULL, en, k);
+                if (dense ? (nw > first || ng > first) : le > lb) {
+                    // chunk and lane prefixes of the sub-segment from the chunk counters
+                    uint32_t off0;
+                    warp_place(chunk_prefixes(cnt8, pre16, c0, CPT), lane, off0);
+                    wl[lane] = off0;
+                    __syncwarp();
+                    auto count = [&](uint32_t kk) -> uint32_t {
+                        return sub_survivors_pre_bits(kk, wl, pre16, bm, CPT, s, warp);
+                    };
+                    int32_t msl = 0;
+                    if (!dense) {
+                        for (uint32_t t = lb + lane; t < le; t += 32) {
+                            const uint32_t e = lbuf[t].x, cv = count(e & 0x7FFFFFFFu);
+                            S += e >> 31 ? (int64_t)cv : -(int64_t)cv;
+                            msl += e >> 31 ? 1 : -1;
+                        }
+                    } else {
+                        const XT xp = shfl_xt(lxp, k);
+                        const double xpd = (double)(uint64_t)xp;
+                        // primes: two leaves a lane a step
+                        const uint32_t *Pk = P + __shfl_sync(FULL, k0_j, k);
+                        uint32_t f = first + lane;
+                        for (; f + step < nw; f += 2 * step) {
+                            const uint32_t m0 = __ldg(Pk + f), m1 = __ldg(Pk + f + step);
+                            S += (int64_t)(count(leaf_bits(xp, xpd, m0)) + count(leaf_bits(xp, xpd, m1)));
+                            msl += 2;
+                        }
+                        if (f < nw) {
+                            S += (int64_t)count(leaf_bits(xp, xpd, __ldg(Pk + f)));
+                            msl += 1;
+                        }
+                        // groups (the next round's are loaded before this round's are answered)
+                        const uint32_t mlo = __shfl_sync(FULL, lmlo, k), mhi = __shfl_sync(FULL, lmhi, k);
+                        const uint64_t i_lo = ((uint64_t)mlo + 1) >> 1, i_hi = ((uint64_t)mhi - 1) >> 1;
+                        uint32_t nbuf = 0;
+                        auto flush = [&] {
+                            __syncwarp();
+                            for (uint32_t t = lane; t < nbuf; t += 32) {
+                                const uint2 e = lbuf[t];
+                                const uint32_t cv = count(leaf_bits(xp, xpd, e.x));
+                                S += e.y ? (int64_t)cv : -(int64_t)cv;
+                                msl += e.y ? 1 : -1;
+                            }
+                            __syncwarp();
+                            nbuf = 0;
+                        };
+                        auto four = [&](uint32_t g) -> int4 {
+                            return g < ng ? __ldg(reinterpret_cast<const int4 *>(MU) + (i_lo >> 2) + g)
+                                          : make_int4(0, 0, 0, 0);
+                        };
+                        int4 next = four(first + lane);
+                        for (uint32_t base = first; base < ng; base += step) {
+                            const uint64_t g4 = (i_lo >> 2) + base + lane;
+                            uint32_t neg = 0, off_l;
+                            uint32_t vm = valid_group(next, g4, i_lo, i_hi, p, &neg);
+                            next = four(base + step + lane);
+                            const uint32_t tot_r = warp_place((uint32_t)__popc(vm), lane, off_l);
+                            if (nbuf + tot_r > kLeafCap) flush();
+                            for (uint32_t t = nbuf + off_l; vm; t++) {
+                                const int kq = __ffs(vm) - 1;
+                                vm &= vm - 1;
+                                lbuf[t] = make_uint2((uint32_t)(2 * (4 * g4 + kq) + 1), (neg >> kq) & 1u);
+                            }
+                            nbuf += tot_r;
+                        }
+                        flush();
+                    }
+                    const int32_t ms = __reduce_add_sync(FULL, msl);
+                    if (lane == k) ar[warp * 32 + k].ms = ms;
+                }
+                // ---- cross off p_b in the sub-segment
+                const uint32_t cleared = cross_off<true>(bm, cnt8, p, __shfl_sync(FULL, lr0, k),
+                                                         __shfl_sync(FULL, li0, k), c0, cw0, CPT, s, CPT * 32 * warp,
+                                                         lane, Lw);
+                tot -= __reduce_add_sync(FULL, cleared);
                 __syncwarp();
-            }
-            // ---- cross off p_b in the sub-segment
-            const uint32_t cleared = cross_off<true>(bm, cnt8, p, __shfl_sync(FULL, lr0, k), __shfl_sync(FULL, li0, k), c0, cw0,
-                                               CPT, s, CPT * 32 * warp, lane, Lw);
-            tot -= __reduce_add_sync(FULL, cleared);
-            __syncwarp();
-            if (lane == k) {
-                mine.cnt = cnt_b;
-                mine.ms = ms_b;
-                mine.job = job_b;
             }
         }
         // ---- combine the warps of the CTA for these 32 levels
-        ar[warp * 32 + lane] = mine;
+        ar[warp * 32 + lane].cnt = mine_cnt;
         __syncthreads();
         if (warp == 0 && lane < nl) {
             const uint32_t b = gb + lane;
@@ -446,11 +474,11 @@ __global__ void __launch_bounds__(512, 2) k_hard(const QD *__restrict__ qd, uint
             for (uint32_t w = 0; w < NW; w++) {
                 const LvlSum e = ar[w * 32 + lane];
                 Sx += (i128)carry * e.ms;
-                if (e.job != 0xFFFFFFFFu) jobs[e.job].carry = carry;
                 carry += e.cnt;
                 msum += e.ms;
             }
-            out_cnt[off + (b - c - 1)] = (uint32_t)carry;
+            // the survivors count once, with the segment's last unit
+            out_cnt[off + (b - c - 1)] = us.part + 1 == us.nparts ? (uint32_t)carry : 0u;
             out_ms[off + (b - c - 1)] = msum;
         }
     }
@@ -458,12 +486,11 @@ __global__ void __launch_bounds__(512, 2) k_hard(const QD *__restrict__ qd, uint
     if (tid == 0) acc_add(acc, q, ACC_HARD, Sb);
 }
 
-// Leaves of the offloaded (segment, level) sets.  A warp takes one unit: 256
+// Leaves of the sets the batch-shared sieve hands over.  A warp takes one unit: 256
 // pi-table entries of prime m (prime-only levels) or 256 groups of 4 odd m
 // read as packed mu*lpf (other levels).  Each leaf's survivor count is the
 // job's carry plus the snapshot's chunk prefix plus popcounts inside the
-// 16-byte chunk; the sums go to the query's hard-leaf accumulator and
-// Sum(-mu) to the level's slot (none when slot = ~0: the carry was complete).
+// 16-byte chunk; the sums go to the query's hard-leaf accumulator.
 template <class XT>
 __global__ void __launch_bounds__(kThreads) k_hard_leaves(const HardJob *__restrict__ jobs,
                                                           const unsigned int *njobs, uint32_t max_jobs,
@@ -471,7 +498,6 @@ __global__ void __launch_bounds__(kThreads) k_hard_leaves(const HardJob *__restr
                                                           const unsigned char *__restrict__ snap,
                                                           uint32_t lbits_sub, const int32_t *__restrict__ MU,
                                                           const cpx_pient *__restrict__ Tpi,
-                                                          int32_t *__restrict__ out_ms,
                                                           unsigned long long *__restrict__ acc)
 {
     const uint32_t n = min(*njobs, max_jobs);
@@ -589,28 +615,40 @@ __global__ void __launch_bounds__(kThreads) k_hard_leaves(const HardJob *__restr
         const i128 Sw = cpx_warp_sum_i128((i128)S);
 #pragma unroll
         for (int dd = 16; dd > 0; dd >>= 1) ms += __shfl_down_sync(FULL, ms, dd);
-        if (lane == 0) {
-            if (ms && J.slot != ~0ull) atomicAdd(out_ms + J.slot, ms);
-            acc_add(acc, J.q, ACC_HARD, Sw + (i128)J.carry * ms);
-        }
+        if (lane == 0) acc_add(acc, J.q, ACC_HARD, Sw + (i128)J.carry * ms);
     }
 }
 
-// B(seg) of every work unit (seg_levels) and its level count max(0, B - c).
+// B(seg) of every work unit (seg_levels) and its level count max(0, B - c);
+// then, one thread per (query, level), the level table of the sieve: x/p, y/p
+// and min(y, x/p^3), which do not depend on the segment.
 template <class XT>
 __global__ void k_hard_plan(const QD *__restrict__ qd, uint32_t Q, const uint64_t *__restrict__ pre_seg,
-                            uint64_t total, const uint32_t *__restrict__ P, uint32_t np,
-                            uint32_t *__restrict__ seg_B, uint64_t *__restrict__ seg_lv)
+                            uint64_t total, const uint64_t *__restrict__ pre_comb, uint64_t total_lv,
+                            const uint32_t *__restrict__ P, uint32_t np, const uint32_t *__restrict__ dense,
+                            uint32_t *__restrict__ seg_B, uint64_t *__restrict__ seg_lv, XT *__restrict__ lvx,
+                            uint2 *__restrict__ lae)
 {
-    const uint64_t u = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (u >= total) return;
-    const uint32_t q = find_q(pre_seg, Q, u);
+    uint64_t u = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (u < total) {
+        const uint32_t q = find_q(pre_seg, Q, u);
+        const QD &d = qd[q];
+        const uint64_t seg = unit_seg(d, dense, u - pre_seg[q]).seg + d.seg0;
+        const uint64_t lo = seg * 2 * (1ull << d.lbits), hi = lo + 2 * (1ull << d.lbits);
+        const uint32_t a = seg_levels<XT>(xload<XT>(d), d.r4, lo, hi, P, np);
+        seg_B[u] = a;
+        seg_lv[u] = a > d.c ? a - d.c : 0;
+        return;
+    }
+    u -= total;
+    if (u >= total_lv) return;
+    const uint32_t q = find_q(pre_comb, Q, u);
     const QD &d = qd[q];
-    const uint64_t seg = u - pre_seg[q] + d.seg0;
-    const uint64_t lo = seg * 2 * (1ull << d.lbits), hi = lo + 2 * (1ull << d.lbits);
-    const uint32_t a = seg_levels<XT>(xload<XT>(d), d.r4, lo, hi, P, np);
-    seg_B[u] = a;
-    seg_lv[u] = a > d.c ? a - d.c : 0;
+    const uint64_t p = P[d.c + (u - pre_comb[q])];
+    const XT xp = cpx_qdiv(xload<XT>(d), p);
+    const XT t3 = cpx_qdiv(xp, p * p);
+    lvx[u] = xp;
+    lae[u] = make_uint2((uint32_t)cpx_udiv_leaf(d.y, p), (uint32_t)(t3 < (XT)d.y ? (uint64_t)t3 : d.y));
 }
 
 // H += sum over segments of carry(seg, b) * msum(seg, b); carry = count of
@@ -618,15 +656,16 @@ __global__ void k_hard_plan(const QD *__restrict__ qd, uint32_t Q, const uint64_
 // segment reaching p_b^2; below p_b^2 the survivors of level b-1 are 1 and the
 // primes from p_b on, so the carry starts at 1 + max(0, pi(lo - 1) - (b - 1))
 // from the pi table and then adds the sieved segments' counts.  One warp per
-// (query, b): its lanes take 32 consecutive segments at a time and a warp
-// scan of their counts gives each segment its carry.  The segments sieving
+// (query, b): its lanes take 32 consecutive units at a time and a warp
+// scan of their counts gives each unit its carry.  The units sieving
 // level b are contiguous from the first one.
 __global__ void k_hard_combine(const QD *__restrict__ qd, uint32_t Q, const uint64_t *__restrict__ pre_comb,
                                uint64_t total, const uint64_t *__restrict__ pre_seg,
                                const uint32_t *__restrict__ seg_B, const uint64_t *__restrict__ seg_off,
                                const uint32_t *__restrict__ cnt, const int32_t *__restrict__ ms, uint64_t cap,
                                const uint32_t *__restrict__ P, const cpx_pient *__restrict__ T,
-                               unsigned long long *__restrict__ acc, HardLevel *__restrict__ lvl_out)
+                               const uint32_t *__restrict__ dense, unsigned long long *__restrict__ acc,
+                               HardLevel *__restrict__ lvl_out)
 {
     const uint64_t u = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t lane = threadIdx.x & 31;
@@ -640,9 +679,11 @@ __global__ void k_hard_combine(const QD *__restrict__ qd, uint32_t Q, const uint
     const uint64_t first = (p * p) / span;  // first segment with hi > p^2
     // the query's segments here are seg0 .. seg0 + n - 1 (all of them unless
     // the query is split over GPUs); carries below the part come from outside
-    const uint64_t g0 = d.seg0, g1 = d.seg0 + (pre_seg[q + 1] - pre_seg[q]);
+    const uint64_t g0 = d.seg0, g1 = d.seg0 + d.nseg;
     const uint64_t fl = first > g0 ? first : g0;
-    const uint64_t s0 = pre_seg[q] + (fl - g0), s1 = pre_seg[q + 1];
+    // units of a segment follow one another, the last of them with its count:
+    // the others' carry is the segment's too
+    const uint64_t s0 = pre_seg[q] + seg_unit(d, dense, fl - g0), s1 = pre_seg[q + 1];
     const bool anchored = first >= g0 && first < g1;
     uint64_t carry = 0;
     if (anchored && first > 0) {
@@ -707,10 +748,10 @@ void launch_hard_leaves(cpx_ctx *ctx, const Plan &pl, uint32_t lbits_sub)
     scan_u64(ctx, pl.job_units, pl.max_jobs + 1);
     if (pl.wide)
         k_hard_leaves<u128><<<(unsigned)ctx->sm_count * 8, kThreads, 0, ctx->stream>>>(
-            pl.jobs, pl.njobs, pl.max_jobs, pl.job_units, pl.snap, lbits_sub, tb.MU, tb.T, pl.hard_ms, pl.acc);
+            pl.jobs, pl.njobs, pl.max_jobs, pl.job_units, pl.snap, lbits_sub, tb.MU, tb.T, pl.acc);
     else
         k_hard_leaves<uint64_t><<<(unsigned)ctx->sm_count * 8, kThreads, 0, ctx->stream>>>(
-            pl.jobs, pl.njobs, pl.max_jobs, pl.job_units, pl.snap, lbits_sub, tb.MU, tb.T, pl.hard_ms, pl.acc);
+            pl.jobs, pl.njobs, pl.max_jobs, pl.job_units, pl.snap, lbits_sub, tb.MU, tb.T, pl.acc);
     CPX_LAUNCH("k_hard_leaves");
     note_launch(ctx);
 }
@@ -718,33 +759,28 @@ void launch_hard_leaves(cpx_ctx *ctx, const Plan &pl, uint32_t lbits_sub)
 template <class XT> static void hard_go(cpx_ctx *ctx, const Plan &pl)
 {
     const Tables &tb = ctx->tab;
-    k_hard_plan<XT><<<(unsigned)((pl.n_seg + 255) / 256), 256, 0, ctx->stream>>>(
-        pl.qd, pl.Q, pl.pre_seg, pl.n_seg, tb.P, (uint32_t)tb.prm_n, pl.seg_B, pl.seg_off);
+    XT *lvx = static_cast<XT *>(pl.lvx);
+    k_hard_plan<XT><<<(unsigned)((pl.n_seg + pl.n_comb + 255) / 256), 256, 0, ctx->stream>>>(
+        pl.qd, pl.Q, pl.pre_seg, pl.n_seg, pl.pre_comb, pl.n_comb, tb.P, (uint32_t)tb.prm_n, pl.dense, pl.seg_B,
+        pl.seg_off, lvx, pl.lae);
     CPX_LAUNCH("k_hard_plan");
     note_launch(ctx);
     scan_u64(ctx, pl.seg_off, pl.n_seg);
     const size_t smem = levels_smem(pl.lbits_max, pl.hard_threads);
-    const uint32_t lbits_sub = pl.lbits_max - (uint32_t)(__builtin_ctz(pl.hard_threads) - 5);
     if (pl.time_hard) CPX_CUDA(cudaEventRecord(ctx->ev_hard0, ctx->stream));
-    if (pl.max_jobs) {
-        CPX_CUDA(cudaMemsetAsync(pl.njobs, 0, sizeof(unsigned int), ctx->stream));
-        CPX_CUDA(cudaMemsetAsync(pl.job_units, 0, (pl.max_jobs + 1) * sizeof(uint64_t), ctx->stream));
-    }
     {
         KSpan ks(ctx, "k_hard");
         k_hard<XT><<<(unsigned)pl.n_seg, pl.hard_threads, smem, ctx->stream>>>(
-            pl.qd, pl.Q, pl.pre_seg, pl.n_seg, pl.seg_B, pl.seg_off, tb.P, tb.MU, tb.T, pl.hard_cnt, pl.hard_ms,
-            pl.hard_entries, pl.acc, pl.lbits_max, pl.jobs, pl.njobs, pl.job_units, pl.snap, pl.max_jobs, lbits_sub,
-            (uint32_t)std::min<uint64_t>(pl.offload_min, 0xFFFFFFFFull));
+            pl.qd, pl.Q, pl.pre_seg, pl.n_seg, pl.seg_B, pl.seg_off, tb.P, tb.MU, tb.T, pl.pre_comb, lvx, pl.lae,
+            pl.dense, pl.hard_cnt, pl.hard_ms, pl.hard_entries, pl.acc, pl.lbits_max);
     }
     CPX_LAUNCH("k_hard");
     note_launch(ctx);
-    if (pl.max_jobs) launch_hard_leaves(ctx, pl, lbits_sub);
     if (pl.time_hard) CPX_CUDA(cudaEventRecord(ctx->ev_hard1, ctx->stream));
     if (pl.n_comb) {
         k_hard_combine<<<(unsigned)((pl.n_comb * 32 + 255) / 256), 256, 0, ctx->stream>>>(
             pl.qd, pl.Q, pl.pre_comb, pl.n_comb, pl.pre_seg, pl.seg_B, pl.seg_off, pl.hard_cnt, pl.hard_ms,
-            pl.hard_entries, tb.P, tb.T, pl.acc, pl.hard_levels);
+            pl.hard_entries, tb.P, tb.T, pl.dense, pl.acc, pl.hard_levels);
         CPX_LAUNCH("k_hard_combine");
         note_launch(ctx);
     }

@@ -154,25 +154,6 @@ __global__ void __launch_bounds__(1024) k_carry_scan(uint32_t nlv, uint32_t c, u
     }
 }
 
-// Quotients n / d by a sub-segment bound d >= 2^13 with rd = 1/d (double,
-// once per warp): for n < 2^64 the quotient is below 2^51, so the truncated
-// product n * rd (relative error at most 3 * 2^-53) is within 1 of it and the
-// sign and size of the remainder n - q d fix it.  128-bit n: exact division.
-struct Recip {
-    uint64_t d;
-    double rd;
-};
-template <class XT> __device__ __forceinline__ XT div_recip(XT n, const Recip &r)
-{
-    if ((u128)n >> 64) return cpx_qdiv(n, r.d);
-    const uint64_t n64 = (uint64_t)n;
-    uint64_t q = __double2ull_rz(__dmul_rn(__ull2double_rn(n64), r.rd));
-    const int64_t rem = (int64_t)(n64 - q * r.d);
-    if (rem < 0) q--;
-    else if ((uint64_t)rem >= r.d) q++;
-    return (XT)q;
-}
-
 // The per-level constants of every query of every group: x/p, y/p and
 // min(y, x/p^3) at index (g nlv + b - c - 1) 32 + slot.  They do not depend
 // on the segment, so k_hard_shared loads them instead of dividing.
@@ -240,12 +221,10 @@ static __device__ __noinline__ bool offload_sets(bool off_j, uint32_t lane, uint
                 J.mlo = prime_j ? qa_j : mlo;
                 J.mhi = mhi;
                 J.lo = lo_w;
-                J.slot = ~0ull;
                 J.nunits = prime_j ? (work / 8 + kJobWords - 1) / kJobWords
                                    : ((((uint64_t)mhi - 1) >> 3) - (((uint64_t)mlo + 1) >> 3) + kJobGroups) / kJobGroups;
                 J.carry = C;
                 J.snap = sn;
-                J.pad = 0;
                 J.xp = (u128)xp;
                 jobs[jb] = J;
                 job_units[jb] = J.nunits;

@@ -12,8 +12,17 @@ constexpr uint32_t kEvCap = 192;
 struct LvlSum {
     uint32_t cnt;
     int32_t ms;
-    uint32_t job;
 };
+
+// leaves a warp gathers before answering them 32 at a time
+constexpr uint32_t kLeafCap = 128;
+
+// bytes of a warp's cleared bits, or of the 16-bit prefixes of its chunks
+__host__ __device__ __forceinline__ size_t ev_bytes(uint32_t lbits, uint32_t threads)
+{
+    const size_t chunks = ((size_t(1) << lbits) / 128) / (threads / 32);
+    return chunks * 2 > kEvCap * 4 ? chunks * 2 : kEvCap * 4;
+}
 
 // shared memory of k_hard
 __host__ __device__ __forceinline__ size_t levels_smem(uint32_t lbits, uint32_t threads)
@@ -25,8 +34,8 @@ __host__ __device__ __forceinline__ size_t levels_smem(uint32_t lbits, uint32_t 
     o += 2 * (threads / 32) * 32 * sizeof(LvlSum);  // per-warp level outputs, double buffered
     o = (o + 15) & ~size_t(15);
     o += 32 * sizeof(i128);                         // reductions
-    o += (threads / 32) * kLeafBuf * 4;             // per-warp gathered leaves
-    o += (threads / 32) * kEvCap * 4;               // per-warp cleared bits
+    o += (threads / 32) * kLeafCap * sizeof(uint2);  // per-warp gathered leaves
+    o += (threads / 32) * ev_bytes(lbits, threads);  // per-warp cleared bits or chunk prefixes
     return o;
 }
 

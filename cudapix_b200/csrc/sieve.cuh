@@ -63,26 +63,6 @@ __host__ __device__ __forceinline__ size_t snap_stride(uint32_t lbits_sub)
 // leaves a warp gathers before answering them 32 at a time
 constexpr uint32_t kLeafBuf = 256;
 
-struct LvlOut {
-    uint32_t cnt;
-    int32_t ms;
-    uint32_t job;
-    uint32_t pad;
-};
-
-__host__ __device__ __forceinline__ size_t hard_smem(uint32_t lbits, uint32_t threads)
-{
-    const size_t L = size_t(1) << lbits;
-    size_t o = L / 8;                                 // bitmap
-    o += ((L / 128) + 15) & ~size_t(15);              // chunk counters
-    o += threads * 4;                                 // lane prefixes
-    o += 2 * (threads / 32) * 32 * sizeof(LvlOut);    // per-warp level outputs, double buffered
-    o = (o + 15) & ~size_t(15);
-    o += 32 * sizeof(i128);                           // reductions
-    o += (threads / 32) * kLeafBuf * 4;               // per-warp gathered leaves
-    return o;
-}
-
 // Pre-sieve of one lane's chunks [c0, c0 + CPT) of the segment starting at lo
 // with p_2 .. p_c (residue masks per 32-bit word); writes the bitmap and the
 // chunk counters and returns the lane's survivors.  Runs once per segment, so
@@ -171,64 +151,23 @@ __device__ __forceinline__ void cross_params(uint64_t p, uint64_t lo_w, uint64_t
     i0 = (m < hi_w) ? (uint32_t)((m - lo_w - 1) >> 1) : 0xFFFFFFFFu;
 }
 
-// Quotients by a warp's sub-segment bounds.  A bound d at or above 2^32 would
-// take the 64-bit hardware division; with rd = 1/d (double, once per warp) the
-// quotient n/d < 2^32 is the truncated product n * rd, whose relative error
-// (three roundings, at most 3 * 2^-53) leaves it within 1 of floor(n/d), fixed
-// by the sign and size of the exact remainder n - q d.
-struct BoundDiv {
+// Quotients n / d by a sub-segment bound d >= 2^13 with rd = 1/d (double,
+// once per warp): for n < 2^64 the quotient is below 2^51, so the truncated
+// product n * rd (relative error at most 3 * 2^-53) is within 1 of it and the
+// sign and size of the remainder n - q d fix it.  128-bit n: exact division.
+struct Recip {
     uint64_t d;
     double rd;
 };
-__device__ __forceinline__ BoundDiv bound_div(uint64_t d)
+template <class XT> __device__ __forceinline__ XT div_recip(XT n, const Recip &r)
 {
-    BoundDiv b;
-    b.d = d;
-    b.rd = (d >> 32) ? 1.0 / (double)d : 0.0;
-    return b;
-}
-template <class XT> __device__ __forceinline__ XT div_bound(XT n, const BoundDiv &b)
-{
-    if (!(b.d >> 32) || ((u128)n >> 64)) return cpx_qdiv(n, b.d);
+    if ((u128)n >> 64) return cpx_qdiv(n, r.d);
     const uint64_t n64 = (uint64_t)n;
-    uint64_t q = __double2ull_rz(__dmul_rn(__ull2double_rn(n64), b.rd));
-    const int64_t r = (int64_t)(n64 - q * b.d);
-    if (r < 0) q--;
-    else if ((uint64_t)r >= b.d) q++;
+    uint64_t q = __double2ull_rz(__dmul_rn(__ull2double_rn(n64), r.rd));
+    const int64_t rem = (int64_t)(n64 - q * r.d);
+    if (rem < 0) q--;
+    else if ((uint64_t)rem >= r.d) q++;
     return (XT)q;
-}
-
-// Parameters of one level (p = p_b) for one warp's sub-segment [lo_w, hi_w):
-// xp = x/p, the candidate range (mlo, mhi] of m (m > y/p, u = xp/m in the
-// sub-segment, m <= x/p^3 for a hard leaf), the residue of lo_w + 1 mod p and
-// the bit of the first odd multiple of p (0xFFFFFFFF: none).  Computed for 32
-// levels at a time, one per lane; out of line to keep the level loop small.
-template <class XT> struct LvlPar {
-    XT xp;
-    uint32_t p, mlo, mhi, r0, i0;
-};
-
-template <class XT>
-static __device__ __noinline__ void level_params(LvlPar<XT> &o, XT x, uint64_t y, uint64_t p, uint64_t lo_w,
-                                                uint64_t hi_w, const BoundDiv &bl, const BoundDiv &bh)
-{
-    const XT xp = cpx_qdiv(x, p);
-    uint64_t mlo = y / p;
-    const XT t1 = div_bound(xp, bh);
-    if (t1 > (XT)mlo) mlo = (uint64_t)t1;
-    uint64_t mhi = y;
-    if (lo_w) {
-        const XT t2 = div_bound(xp, bl);
-        if (t2 < (XT)mhi) mhi = (uint64_t)t2;
-    }
-    const XT t3 = cpx_qdiv(xp, p * p);  // hard leaves only: m <= x/p^3
-    if (t3 < (XT)mhi) mhi = (uint64_t)t3;
-    if (mhi < mlo) mhi = mlo;
-    o.p = (uint32_t)p;
-    o.xp = xp;
-    o.mlo = (uint32_t)mlo;
-    o.mhi = (uint32_t)mhi;
-    cross_params(p, lo_w, hi_w, o.r0, o.i0);
 }
 
 // Crosses p off one warp's sub-segment of Lw bits (chunks [base_ch, base_ch +
@@ -362,14 +301,11 @@ __device__ __forceinline__ uint32_t chunk_survivors(uint4 v4, uint32_t jb)
     return __popc(v4.x & m0) + __popc(v4.y & m1) + __popc(v4.z & m2) + __popc(v4.w & m3);
 }
 
-// Survivors of a warp's sub-segment [lo_w, lo_w + 2 Lw) with n <= uu, uu in
-// [lo_w, hi_w), from the lane prefixes wl[] of the sub-segment, the chunk
-// counters and the chunk's popcounts.
-__device__ __forceinline__ uint32_t sub_survivors(uint64_t uu, uint64_t lo_w, const uint32_t *wl, const uint8_t *cnt8,
-                                                  const uint32_t *bm, uint32_t CPT, int s, uint32_t warp)
+// Survivors among bits [0, kk) of a warp's sub-segment, from the lane prefixes
+// wl[] of the sub-segment, the chunk counters and the chunk's popcounts.
+__device__ __forceinline__ uint32_t sub_survivors_bits(uint32_t kk, const uint32_t *wl, const uint8_t *cnt8,
+                                                       const uint32_t *bm, uint32_t CPT, int s, uint32_t warp)
 {
-    // bits [0, kk) of the sub-segment; uu - lo_w < 2^21, so its low 32 bits suffice
-    const uint32_t kk = ((uint32_t)uu - (uint32_t)lo_w + 1u) >> 1;
     if (!kk) return 0u;
     const uint32_t jb = kk - 1, w = jb >> 5;
     const uint32_t chs = w >> 2, ow = chs >> s;  // chunk in the sub-segment, owning lane
@@ -424,19 +360,24 @@ __device__ __forceinline__ uint32_t chunk_prefixes(const uint8_t *cnt8, uint16_t
     return run;
 }
 
-// sub_survivors from the chunk prefixes of chunk_prefixes: the owner lane's
-// prefix, the chunk's prefix within the owner and the chunk's popcounts.
-__device__ __forceinline__ uint32_t sub_survivors_pre(uint64_t uu, uint64_t lo_w, const uint32_t *wl,
-                                                      const uint16_t *pre16, const uint32_t *bm, uint32_t CPT, int s,
-                                                      uint32_t warp)
+// sub_survivors_bits from the chunk prefixes of chunk_prefixes: the owner
+// lane's prefix, the chunk's prefix within the owner and the chunk's popcounts.
+__device__ __forceinline__ uint32_t sub_survivors_pre_bits(uint32_t kk, const uint32_t *wl, const uint16_t *pre16,
+                                                           const uint32_t *bm, uint32_t CPT, int s, uint32_t warp)
 {
-    // bits [0, kk) of the sub-segment; uu - lo_w < 2^21, so its low 32 bits suffice
-    const uint32_t kk = ((uint32_t)uu - (uint32_t)lo_w + 1u) >> 1;
     if (!kk) return 0u;
     const uint32_t jb = kk - 1;
     const uint32_t chs = jb >> 7;               // chunk in the sub-segment
     const uint32_t ch = chs + CPT * 32 * warp;  // chunk in the segment
     return wl[chs >> s] + pre16[ch] + chunk_survivors(reinterpret_cast<const uint4 *>(bm)[swz(ch, s)], jb);
+}
+// Survivors of a warp's sub-segment [lo_w, lo_w + 2 Lw) with n <= uu, uu in
+// [lo_w, hi_w): bits [0, kk) (uu - lo_w < 2^21, so its low 32 bits suffice).
+__device__ __forceinline__ uint32_t sub_survivors_pre(uint64_t uu, uint64_t lo_w, const uint32_t *wl,
+                                                      const uint16_t *pre16, const uint32_t *bm, uint32_t CPT, int s,
+                                                      uint32_t warp)
+{
+    return sub_survivors_pre_bits(((uint32_t)uu - (uint32_t)lo_w + 1u) >> 1, wl, pre16, bm, CPT, s, warp);
 }
 
 // B(seg) = pi(min(r4, isqrt((x - 1) / lo), isqrt(hi - 1))): the levels b a

@@ -15,6 +15,8 @@ struct __align__(16) QD {
     uint32_t p2win;                 // P2 by pi-table windows over [sqrt x, z] (z beyond the table)
     uint32_t piy;                   // pi(y) when P2 walks the prime list (Plan::p2_primes)
     uint64_t seg0;                  // first hard-leaf segment (a part of a query split over GPUs)
+    uint32_t dense_segs, dense_off; // first segments whose leaves are split over several units, and where
+                                    // Plan::dense holds the units before each (dense_segs + 1 entries)
 };
 
 // Per level b of a query's part: survivors of level b-1 over its segments,
@@ -35,21 +37,19 @@ struct __align__(16) EasyLvl {
     uint64_t i_lo, i_hi, i_base, unit0;
 };
 
-// A heavy (sub-segment, level) leaf set handed from a sieve kernel to
+// A heavy (sub-segment, level) leaf set handed from the batch-shared sieve to
 // k_hard_leaves: the sub-segment's bitmap and per-chunk survivor prefixes at
 // level b-1 sit in snapshot slot `snap` (one slot can serve the sets of
 // several queries); the leaves are m in (mlo, mhi] (prime m only when
 // kind = 1).  nunits counts its k_hard_leaves work units; their offsets are
-// the scanned job-unit array.  `slot` is the level output that receives
-// Sum(-mu), ~0 when `carry` already counts every survivor below the
-// sub-segment.
+// the scanned job-unit array.  `carry` counts every survivor of level b-1
+// below the sub-segment.
 struct __align__(16) HardJob {
     uint32_t q, b, p, kind;
-    uint64_t mlo, mhi, lo, slot;  // lo: first number of the warp's sub-segment
-    uint64_t nunits;              // k_hard_leaves work units
-    uint64_t carry;               // survivors of level b-1 below the sub-segment (in its segment, or all)
-    uint64_t snap;                // snapshot slot
-    uint64_t pad;
+    uint64_t mlo, mhi, lo;  // lo: first number of the warp's sub-segment
+    uint64_t nunits;        // k_hard_leaves work units
+    uint64_t carry;         // survivors of level b-1 below the sub-segment
+    uint64_t snap;          // snapshot slot
     u128 xp;
 };
 
@@ -92,7 +92,11 @@ struct Plan {
     int32_t *hard_ms = nullptr;
     unsigned long long *acc = nullptr;
     unsigned int *ticket = nullptr;
-    // heavy hard-leaf sets offloaded from k_hard
+    // per (query, level) of the lone-query sieve (pre_comb): x/p and {y/p, min(y, x/p^3)}
+    void *lvx = nullptr;
+    uint2 *lae = nullptr;
+    const uint32_t *dense = nullptr;  // units before each dense segment, per query (QD::dense_off)
+    // heavy hard-leaf sets offloaded from k_hard_shared
     HardJob *jobs = nullptr;
     unsigned int *njobs = nullptr;   // device counter
     uint64_t *job_units = nullptr;   // max_jobs + 1 work-unit counts, scanned into offsets

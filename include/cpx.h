@@ -84,9 +84,11 @@ int cpx_mem_info(cpx_ctx *ctx, uint64_t *free_bytes, uint64_t *total_bytes);
 /* hard-leaf sieve tuning: segment = 2^log2_bits odd numbers (15..20),
  * threads per CTA in {128, 256, 512}. */
 int cpx_set_hard_params(cpx_ctx *ctx, uint32_t log2_bits, uint32_t threads);
-/* a (sub-segment, level) of the hard-leaf sieve with at least min_candidates
- * candidate m is answered by a separate GPU-wide leaf kernel from a snapshot
- * of the sub-segment; 0 answers every leaf inside the sieve (default 1024) */
+/* a (sub-segment, level) of the batch-shared hard-leaf sieve with at least
+ * min_candidates candidate m is answered by a separate GPU-wide leaf kernel
+ * from a snapshot of the sub-segment; 0 answers every leaf inside the sieve
+ * (default 1024).  One sieve per query splits its densest segments over
+ * several CTAs instead, whatever this value. */
 int cpx_set_hard_offload(cpx_ctx *ctx, uint32_t min_candidates);
 /* Batches share one hard-leaf sieve between their queries: the survivor
  * counts of one sweep give every (sub-segment, level) its carry, and each
