@@ -10,6 +10,7 @@
 #include <algorithm>
 
 #include "misc.h"
+#include "sieve_block.cuh"
 
 namespace cpx {
 
@@ -72,20 +73,124 @@ __device__ __forceinline__ uint64_t odd_rel(const cpx_pient *__restrict__ T, uin
     return e.y + __popcll(e.x & ((2ull << j) - 1));
 }
 
-// out[k] = pi(base + 2k - 1) - pi(base - 1)   (k = 0 -> 0); base even
-__global__ void k_pi_window(const cpx_pient *__restrict__ T, uint64_t w0, uint64_t base, uint64_t K,
+// out[k] = pi(base + 2k - 1) - pi(base - 1)   (k = 0 -> 0); base even.  Four
+// outputs a thread, one 16-byte store (vec: out is 16-byte aligned); they lie
+// in one table entry or two.  5e7 outputs: 194 us
+// one output a thread, 119 us so (the 200 MB written take 31).
+__global__ void k_pi_window(const cpx_pient *__restrict__ T, uint64_t w0, uint64_t base, uint64_t K, int vec,
                             uint32_t *__restrict__ out)
 {
-    const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= K) return;
-    if (k == 0) {
-        out[0] = 0;
+    const uint64_t k0 = 4 * ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x);
+    if (k0 >= K) return;
+    const uint64_t below = base ? odd_rel(T, w0, base - 1) : 0;
+    uint64_t w = ~0ull;
+    ulonglong2 e = make_ulonglong2(0, 0);
+    uint32_t o[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        const uint64_t k = k0 + j;
+        o[j] = 0;
+        if (k == 0 || k >= K) continue;
+        const uint64_t n = base + 2 * k - 1;
+        if (((n - 1) >> 7) != w) {
+            w = (n - 1) >> 7;
+            e = __ldg(reinterpret_cast<const ulonglong2 *>(T) + (w - w0));
+        }
+        uint64_t v = e.y + __popcll(e.x & ((2ull << (((n - 1) & 127) >> 1)) - 1)) - below;
+        if (base <= 2 && n >= 2) v += 1;  // the prime 2
+        o[j] = (uint32_t)v;
+    }
+    if (vec && k0 + 4 <= K) {
+        reinterpret_cast<uint4 *>(out)[k0 >> 2] = make_uint4(o[0], o[1], o[2], o[3]);
+    } else {
+        for (int j = 0; j < 4 && k0 + j < K; j++) out[k0 + j] = o[j];
+    }
+}
+
+static void launch_pi_window(cpx_ctx *ctx, const cpx_pient *T, uint64_t w0, uint64_t base, uint64_t K, uint32_t *out)
+{
+    const int vec = (reinterpret_cast<uintptr_t>(out) & 15) == 0;
+    k_pi_window<<<(unsigned)((K + 1023) / 1024), 256, 0, ctx->stream>>>(T, w0, base, K, vec, out);
+    CPX_LAUNCH("k_pi_window");
+    note_launch(ctx);
+}
+
+// Sieves CTA blocks of MUL x 2^18 odd numbers from lo0 (a multiple of 128) and
+// adds the odd n of [nlo, nmax] that are left to *count; with words, writes
+// them as 64-bit words (bit j of word w: lo0 + 128 w + 2j + 1) instead.
+// PRIME: the primes; else the n that no P[1] .. P[np - 1] divides.
+// Issue and shared-memory atomics bound it.  The primes of 1e10 numbers at
+// 1e12: 11.3 ms as a pi table, 3.65 ms so; phi(1e10, 100), formerly with a
+// division per word and prime below 64: 11.1 -> 1.03 ms.
+template <bool PRIME, int MUL>
+__global__ void __launch_bounds__(256 * MUL) k_block_sieve(uint64_t lo0, const uint32_t *__restrict__ P, uint32_t np,
+                                                           uint64_t nlo, uint64_t nmax, uint64_t *__restrict__ words,
+                                                           uint64_t nwords, unsigned long long *__restrict__ count)
+{
+    constexpr uint32_t NT = 256 * MUL;
+    extern __shared__ uint32_t bm[];  // the bitmap, then the patterns
+    const uint32_t tid = threadIdx.x;
+    const uint64_t lo = lo0 + 2048ull * NT * blockIdx.x;
+    sieve_block<PRIME, NT>(bm, bm + NT * 32, lo, P, np);
+    if (words) {
+        const uint64_t *bm64 = reinterpret_cast<const uint64_t *>(bm);
+        for (uint32_t w = tid; w < NT * 16; w += NT) {
+            const uint64_t gw = 16ull * NT * blockIdx.x + w;
+            if (gw < nwords) words[gw] = bm64[w];
+        }
         return;
     }
-    const uint64_t n = base + 2 * k - 1;
-    uint64_t v = odd_rel(T, w0, n) - (base ? odd_rel(T, w0, base - 1) : 0);
-    if (base <= 2 && n >= 2) v += 1;  // the prime 2
-    out[k] = (uint32_t)v;
+    uint32_t s = 0;
+    const bool inside = lo >= nlo && nmax - lo >= 2048ull * NT;
+    for (uint32_t w = tid; w < NT * 32; w += NT) {
+        uint32_t b = bm[w];
+        if (!inside) {
+            // bit k is n = base + 2k + 1
+            const uint64_t base = lo + 64ull * w;
+            if (base >= nmax || base + 64 <= nlo) continue;
+            const uint64_t kmax = (nmax - base - 1) >> 1, kmin = nlo > base ? (nlo - base) >> 1 : 0;
+            if (kmax < 31) b &= (2u << kmax) - 1u;
+            if (kmin > 31) continue;
+            b &= ~0u << kmin;
+        }
+        s += __popc(b);
+    }
+    s = __reduce_add_sync(0xffffffffu, s);
+    if ((tid & 31) == 0 && s) atomicAdd(count, (unsigned long long)s);
+}
+
+// the sieve above over the odd n of [nlo, nmax] (blocks from nlo rounded down to
+// a multiple of 128).  Launches only.  Blocks of 2^20 numbers, three CTAs an SM
+// whose phases overlap, when they fill the GPU; of 2^21 when the sieving primes
+// are many, as a CTA pays each one's start once for all its numbers (phi(1e10,
+// 100) 1.03 against 1.11 ms, primes of 1e10 numbers at 1e10 0.25 against 0.29 a
+// billion, at 1e12 4.24 against 3.80); else of 2^19.
+template <bool PRIME>
+static void launch_block_sieve(cpx_ctx *ctx, uint32_t np, uint64_t nlo, uint64_t nmax, uint64_t *words, uint64_t nwords,
+                               unsigned long long *count)
+{
+    const uint64_t lo0 = nlo & ~uint64_t(127);
+    constexpr uint64_t kMaxGrid = 1u << 30;
+    auto go = [&](auto kern, uint32_t nt, size_t smem) {
+        const uint64_t span = 2048ull * nt, nblk = (nmax - lo0) / span + 1;
+        for (uint64_t b = 0; b < nblk; b += kMaxGrid) {
+            kern<<<(unsigned)std::min(nblk - b, kMaxGrid), nt, smem, ctx->stream>>>(
+                lo0 + b * span, ctx->tab.P, np, nlo, nmax, words, nwords, count);
+            CPX_LAUNCH("k_block_sieve");
+            note_launch(ctx);
+        }
+    };
+    const uint64_t blocks = (nmax - lo0) >> 20, sms = (uint64_t)ctx->sm_count;
+    const bool many = PRIME ? nmax >> 32 >= 4 : np > 20000;  // primes beyond about 2^17
+    if (many && blocks >= 4 * sms) {
+        raise_smem<k_block_sieve<PRIME, 4>>(ctx, sieve_block_smem(1024));
+        go(k_block_sieve<PRIME, 4>, 1024, sieve_block_smem(1024));
+    } else if (blocks >= 3 * sms) {
+        raise_smem<k_block_sieve<PRIME, 2>>(ctx, sieve_block_smem(512));
+        go(k_block_sieve<PRIME, 2>, 512, sieve_block_smem(512));
+    } else {
+        go(k_block_sieve<PRIME, 1>, 256, sieve_block_smem(256));
+    }
 }
 
 // count of primes in [lo, hi) from a window table covering them
@@ -97,13 +202,26 @@ __global__ void k_count_window(const cpx_pient *__restrict__ T, uint64_t w0, uin
     atomicAdd(out, (unsigned long long)v);
 }
 
+// the table entries of a window over [lo, hi), and the primes that sieve it
+static void window_words(uint64_t lo, uint64_t hi, uint64_t &w0, uint64_t &nwords)
+{
+    w0 = lo / 128;
+    const uint64_t w1 = (hi + 127) / 128 + 1;
+    nwords = (w1 - w0 + kTabSegWords - 1) / kTabSegWords * kTabSegWords;
+}
+static uint64_t window_prime_bound(uint64_t lo, uint64_t hi)
+{
+    uint64_t w0, nwords;
+    window_words(lo, hi, w0, nwords);
+    return cpx_isqrt((u128)((w0 + nwords) * 128)) + 2;
+}
+
 // Window table over [A, B) with A = 128*w0 <= lo and B >= hi into ctx->b_win.
 static cpx_pient *window_table(cpx_ctx *ctx, uint64_t lo, uint64_t hi, uint64_t *w0_out)
 {
-    const uint64_t w0 = lo / 128;
-    const uint64_t w1 = (hi + 127) / 128 + 1;
-    const uint64_t nwords = (w1 - w0 + kTabSegWords - 1) / kTabSegWords * kTabSegWords;
-    ensure_primes(ctx, cpx_isqrt((u128)((w0 + nwords) * 128)) + 2);
+    uint64_t w0, nwords;
+    window_words(lo, hi, w0, nwords);
+    ensure_primes(ctx, window_prime_bound(lo, hi));
     cpx_pient *T = ctx->b_win.as<cpx_pient>(nwords);
     build_pitable_window(ctx, w0, nwords, T);
     *w0_out = w0;
@@ -118,25 +236,25 @@ uint64_t count_primes(cpx_ctx *ctx, uint64_t lo, uint64_t hi)
     unsigned long long *d = ctx->b_small.as<unsigned long long>(8) + 1;
     CPX_CUDA(cudaMemsetAsync(d, 0, 8, ctx->stream));
     const Tables &tb = ctx->tab;
+    uint64_t two = 0;  // the prime 2, which no bitmap holds
     if (tb.T && hi - 1 <= tb.tab_n) {
         k_count_window<<<1, 1, 0, ctx->stream>>>(tb.T, 0, lo, hi, d);
         CPX_LAUNCH("k_count_window");
         note_launch(ctx);
     } else {
+        // sieved and counted block by block, without a table
+        two = lo <= 2 && 2 < hi;
         for (uint64_t a = lo; a < hi;) {
             const uint64_t b = (hi - a > kWindowSpan) ? a + kWindowSpan : hi;
-            uint64_t w0;
-            cpx_pient *T = window_table(ctx, a, b, &w0);
-            k_count_window<<<1, 1, 0, ctx->stream>>>(T, w0, a, b, d);
-            CPX_LAUNCH("k_count_window");
-            note_launch(ctx);
+            ensure_primes(ctx, window_prime_bound(a, b));
+            launch_block_sieve<true>(ctx, (uint32_t)tb.prm_n, a, b - 1, nullptr, 0, d);
             a = b;
         }
     }
     unsigned long long h = 0;
     CPX_CUDA(cudaMemcpyAsync(&h, d, 8, cudaMemcpyDeviceToHost, ctx->stream));
     CPX_CUDA(cudaStreamSynchronize(ctx->stream));
-    return h;
+    return h + two;
 }
 
 void pitable_window(cpx_ctx *ctx, uint64_t base, uint64_t range, uint32_t *d_out, uint64_t *pi_base)
@@ -149,9 +267,7 @@ void pitable_window(cpx_ctx *ctx, uint64_t base, uint64_t range, uint32_t *d_out
     uint64_t w0 = 0;
     if (tb.T && top <= tb.tab_n) T = tb.T;
     else T = window_table(ctx, base, top, &w0);
-    k_pi_window<<<(unsigned)((K + 255) / 256), 256, 0, ctx->stream>>>(T, w0, base, K, d_out);
-    CPX_LAUNCH("k_pi_window");
-    note_launch(ctx);
+    launch_pi_window(ctx, T, w0, base, K, d_out);
     CPX_CUDA(cudaStreamSynchronize(ctx->stream));
     if (pi_base) *pi_base = base ? count_primes(ctx, 0, base) : 0;
 }
@@ -164,9 +280,7 @@ uint32_t *pitable_dense(cpx_ctx *ctx, uint64_t hi)
     CPX_CUDA(cudaMalloc(&out, std::max<uint64_t>(K, 1) * 4));
     if (K) {
         ensure_pitable(ctx, hi + 2);
-        k_pi_window<<<(unsigned)((K + 255) / 256), 256, 0, ctx->stream>>>(ctx->tab.T, 0, 0, K, out);
-        CPX_LAUNCH("k_pi_window");
-        note_launch(ctx);
+        launch_pi_window(ctx, ctx->tab.T, 0, 0, K, out);
         CPX_CUDA(cudaStreamSynchronize(ctx->stream));
     }
     return out;
@@ -257,73 +371,6 @@ uint64_t extract_window(cpx_ctx *ctx, const cpx_pient *T, uint64_t w0, uint64_t 
 }
 
 // ------------------------------------------------------------------ phi sieve
-// Odd-only bitmap of [2*64*w0, ...): bit set iff n has no prime factor among
-// p_2 .. p_a (n = 1 stays set).  One CTA per 2^18 odd numbers; p < 64 by
-// residue masks per word, larger p by strided shared-memory atomicAnd.
-// Either writes the words (out) or adds popcount(n <= nmax) to *count.
-constexpr uint32_t kPhiSegW = 4096;  // 64-bit words per CTA
-
-__global__ void __launch_bounds__(256) k_phi_sieve(uint64_t w0, const uint32_t *__restrict__ P, uint32_t a,
-                                                   uint64_t *__restrict__ out, uint64_t nwords_out, uint64_t nmax,
-                                                   unsigned long long *__restrict__ count)
-{
-    __shared__ uint32_t bm[2 * kPhiSegW];
-    const uint32_t tid = threadIdx.x;
-    const uint64_t wbase = w0 + (uint64_t)blockIdx.x * kPhiSegW;  // in 64-bit words
-    const uint64_t lo = wbase * 128;
-    const uint64_t hi = lo + 128ull * kPhiSegW;
-    constexpr uint32_t NB = 2 * kPhiSegW * 32;
-    for (uint32_t w = tid; w < 2 * kPhiSegW; w += 256) {
-        // 32-bit word w covers n = lo + 64 w + 2k + 1
-        uint32_t m = 0;
-        for (uint32_t i = 1; i < a; i++) {
-            const uint32_t p = P[i];
-            if (p >= 64) break;
-            const uint32_t r = (uint32_t)((lo + 64ull * w + 1) % p);
-            const uint32_t k0 = (r == 0) ? 0u : ((r & 1u) ? (p - r) >> 1 : p - (r >> 1));
-            for (uint32_t k = k0; k < 32; k += p) m |= 1u << k;
-        }
-        bm[w] = ~m;
-    }
-    __syncthreads();
-    for (uint32_t i = 1; i < a; i++) {
-        const uint64_t p = P[i];
-        if (p < 64) continue;
-        if (p >= hi) break;
-        const uint64_t r = (lo + 1) % p;
-        uint64_t m = lo + 1 + (r ? p - r : 0);
-        if ((m & 1) == 0) m += p;
-        if (m >= hi) continue;
-        const uint64_t i0 = (m - lo - 1) >> 1;
-        for (uint64_t bi = i0 + tid * p; bi < NB; bi += 256 * p) atomicAnd(&bm[bi >> 5], ~(1u << (bi & 31)));
-    }
-    __syncthreads();
-    const uint64_t *bm64 = reinterpret_cast<const uint64_t *>(bm);
-    if (out) {
-        for (uint32_t w = tid; w < kPhiSegW; w += 256) {
-            const uint64_t gw = wbase + w;
-            if (gw - w0 < nwords_out) out[gw - w0] = bm64[w];
-        }
-    }
-    if (count) {
-        unsigned long long s = 0;
-        for (uint32_t w = tid; w < kPhiSegW; w += 256) {
-            const uint64_t base = 128 * (wbase + w);
-            if (base + 1 > nmax) continue;
-            uint64_t b = bm64[w];
-            const uint64_t lim = nmax - base - 1;  // bit j valid iff 2j <= lim
-            if (lim < 127) {
-                const uint32_t j = (uint32_t)(lim >> 1);
-                b &= (2ull << j) - 1;
-            }
-            s += __popcll(b);
-        }
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) s += __shfl_down_sync(0xffffffffu, s, d);
-        if ((tid & 31) == 0 && s) atomicAdd(count, s);
-    }
-}
-
 static void ensure_nth_prime(cpx_ctx *ctx, uint32_t a)
 {
     uint64_t pm = std::max<uint64_t>(ctx->tab.prm_max, 1 << 16);
@@ -338,16 +385,9 @@ uint64_t phi_count(cpx_ctx *ctx, uint64_t x, uint32_t a)
 {
     if (a == 0 || x == 0) return x;
     ensure_nth_prime(ctx, a);
-    const uint64_t nw = x / 128 + 1;
-    const uint64_t nseg = (nw + kPhiSegW - 1) / kPhiSegW;
     unsigned long long *d = ctx->b_small.as<unsigned long long>(8) + 3;
     CPX_CUDA(cudaMemsetAsync(d, 0, 8, ctx->stream));
-    for (uint64_t s0 = 0; s0 < nseg; s0 += 1u << 30) {
-        const uint64_t ns = std::min<uint64_t>(nseg - s0, 1u << 30);
-        k_phi_sieve<<<(unsigned)ns, 256, 0, ctx->stream>>>(s0 * kPhiSegW, ctx->tab.P, a, nullptr, 0, x, d);
-        CPX_LAUNCH("k_phi_sieve");
-        note_launch(ctx);
-    }
+    launch_block_sieve<false>(ctx, a, 0, x, nullptr, 0, d);
     unsigned long long h = 0;
     CPX_CUDA(cudaMemcpyAsync(&h, d, 8, cudaMemcpyDeviceToHost, ctx->stream));
     CPX_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -377,11 +417,8 @@ __global__ void k_popc_words(const uint64_t *__restrict__ words, uint64_t n, uin
 void phi_bits(cpx_ctx *ctx, uint64_t nwords, uint32_t a, uint64_t *words)
 {
     if (a >= 1) ensure_nth_prime(ctx, a);
-    const uint64_t nseg = (nwords + kPhiSegW - 1) / kPhiSegW;
-    if (nseg > 0x7FFFFFFFull) fail(CPX_ERANGE, "phi sieve too large");
-    k_phi_sieve<<<(unsigned)nseg, 256, 0, ctx->stream>>>(0, ctx->tab.P, a == 0 ? 1 : a, words, nwords, 0, nullptr);
-    CPX_LAUNCH("k_phi_sieve");
-    note_launch(ctx);
+    if (nwords > (0x7FFFFFFFull << 12)) fail(CPX_ERANGE, "phi sieve too large");
+    launch_block_sieve<false>(ctx, a == 0 ? 1 : a, 0, 128 * nwords - 1, words, nwords, nullptr);
 }
 
 void counts_from_bits(cpx_ctx *ctx, const uint64_t *words, uint64_t nwords, uint64_t nbits, int inclusive,

@@ -14,7 +14,7 @@
 #include <mutex>
 #include <algorithm>
 
-#include "cpx_internal.h"
+#include "sieve_block.cuh"
 
 namespace cpx {
 
@@ -158,13 +158,6 @@ __global__ void __launch_bounds__(512) k_trial_table(cpx_pient *T)
 
 // ------------------------------------------------------ segmented prime sieve
 
-// Odd primes 3..31 are removed with per-word residue masks; 37..8191 by all
-// threads together (one prime at a time, strided multiples, shared-memory
-// atomicAnd); larger primes one per thread.
-constexpr int kSmallCnt = 10;  // 3 .. 31
-__constant__ uint32_t c_small[kSmallCnt] = {3, 5, 7, 11, 13, 17, 19, 23, 29, 31};
-constexpr uint32_t kCoopMax = 1017;  // primes in [37, 8192)
-
 __device__ __forceinline__ uint32_t first_odd_multiple_idx(uint64_t lo, uint64_t hi, uint64_t p,
                                                             bool from_square)
 {
@@ -181,111 +174,45 @@ __device__ __forceinline__ uint32_t first_odd_multiple_idx(uint64_t lo, uint64_t
 
 // One CTA sieves MUL table blocks of kTabSegWords entries (2^18 odd numbers
 // each) with MUL x 256 threads and writes, per block, its entries (prefix
-// relative to the block) and its total.  A CTA pays the start offset of every
-// sieving prime once for all its numbers, so MUL = 4 (2^20 odd numbers, 128 KB
-// of dynamic shared memory) spreads that cost over four times the numbers
-// for the large windows of P2 beyond the resident table.
+// relative to the block) and its total.  A CTA pays the start of every sieving
+// prime once for all its numbers, so MUL = 4 (2^20 odd numbers, 139 KB of
+// shared memory) spreads that cost over four times the numbers.
+// Shared-memory atomics and issue bound it, not the 16 bytes per 128 numbers it
+// writes: the table of pi(1e17), 4.5e9 numbers, took 2.78 ms with residue masks
+// to 31 and every thread on every prime to 8191, 0.97 ms now.
 template <int MUL>
-__global__ void __launch_bounds__(kThreads * MUL) k_sieve_table(uint64_t w0, const uint32_t *__restrict__ sp,
-                                                                uint32_t nsp, uint32_t ncoop,
-                                                                cpx_pient *__restrict__ T,
+__global__ void __launch_bounds__(kThreads * MUL) k_sieve_table(uint64_t w0, const uint32_t *__restrict__ P,
+                                                                uint32_t np, cpx_pient *__restrict__ T,
                                                                 uint64_t *__restrict__ segtot)
 {
     constexpr uint32_t NT = kThreads * MUL;
-    constexpr uint32_t NW32 = kTabSegWords * 2 * MUL;  // 8192 MUL words = 2^18 MUL bits
-    constexpr uint32_t NBITS = NW32 * 32;
-    extern __shared__ uint32_t bm[];  // NW32 words
-    __shared__ uint32_t off[kCoopMax];
-    __shared__ uint32_t pat[160];
-    __shared__ uint32_t lomod[kSmallCnt];
-    __shared__ uint64_t wsum[NT / 32];
+    extern __shared__ uint32_t bm[];  // the bitmap, then the patterns
+    __shared__ uint32_t wsum[NT / 32];
     const uint32_t tid = threadIdx.x;
     const uint64_t wbase = w0 + (uint64_t)blockIdx.x * kTabSegWords * MUL;
-    const uint64_t lo = wbase * 128, hi = lo + kTabSegNumbers * MUL;
-
-    // residue masks: pat[o_p + r] = bits k < 32 with (r + 2k) % p == 0
-    if (tid < 158) {
-        uint32_t o = 0, i = 0;
-        while (tid >= o + c_small[i]) o += c_small[i++];
-        uint32_t p = c_small[i], r = tid - o, m = 0;
-        for (uint32_t k = 0; k < 32; k++)
-            if ((r + 2 * k) % p == 0) m |= 1u << k;
-        pat[tid] = m;
-    }
-    if (tid < kSmallCnt) lomod[tid] = (uint32_t)((lo + 1) % c_small[tid]);
-    for (uint32_t k = tid; k < ncoop; k += NT)
-        off[k] = first_odd_multiple_idx(lo, hi, sp[k], true);
-    __syncthreads();
-
-    {
-        uint32_t r[kSmallCnt], step[kSmallCnt], base[kSmallCnt];
-        uint32_t o = 0;
-#pragma unroll
-        for (int i = 0; i < kSmallCnt; i++) {
-            const uint32_t p = c_small[i];
-            r[i] = (lomod[i] + (64u * tid) % p) % p;
-            step[i] = (64u * NT) % p;
-            base[i] = o;
-            o += p;
-        }
-        for (uint32_t w = tid; w < NW32; w += NT) {
-            uint32_t m = 0;
-#pragma unroll
-            for (int i = 0; i < kSmallCnt; i++) {
-                m |= pat[base[i] + r[i]];
-                r[i] += step[i];
-                if (r[i] >= c_small[i]) r[i] -= c_small[i];
-            }
-            bm[w] = ~m;
-        }
-    }
-    __syncthreads();
-
-    for (uint32_t k = 0; k < ncoop; k++) {
-        const uint32_t i0 = off[k];
-        if (i0 == 0xFFFFFFFFu) continue;
-        const uint32_t p = sp[k];
-        for (uint32_t i = i0 + tid * p; i < NBITS; i += NT * p) atomicAnd(&bm[i >> 5], ~(1u << (i & 31)));
-    }
-    for (uint32_t k = ncoop + tid; k < nsp; k += NT) {
-        const uint64_t p = sp[k];
-        if (p * p >= hi) break;
-        uint32_t i0 = first_odd_multiple_idx(lo, hi, p, true);
-        if (i0 == 0xFFFFFFFFu) continue;
-        for (uint64_t i = i0; i < NBITS; i += p) atomicAnd(&bm[i >> 5], ~(1u << (i & 31)));
-    }
-    __syncthreads();
-    if (lo == 0 && tid == 0) {
-        // 1 is not prime; the residue masks removed 3..31 themselves
-        uint32_t v = bm[0] & ~1u;
-        v |= (1u << 1) | (1u << 2) | (1u << 3) | (1u << 5) | (1u << 6) | (1u << 8) | (1u << 9) |
-             (1u << 11) | (1u << 14) | (1u << 15);
-        bm[0] = v;
-    }
-    __syncthreads();
+    sieve_block<true, NT>(bm, bm + NT * 32, wbase * 128, P, np);
 
     // per-warp popcount totals, then a warp-level scan writing {bits, prefix}
     // with prefixes relative to the warp's table block (8 warps a block)
     const int lane = tid & 31, wi = tid >> 5;
     const uint64_t *bm64 = reinterpret_cast<const uint64_t *>(bm);
     constexpr uint32_t PER_WARP = kTabSegWords / (kThreads / 32);  // 512
-    uint64_t s = 0;
+    uint32_t s = 0;
     for (uint32_t i = 0; i < PER_WARP / 32; i++) s += __popcll(bm64[wi * PER_WARP + 32 * i + lane]);
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) s += __shfl_down_sync(0xffffffffu, s, d);
+    s = __reduce_add_sync(0xffffffffu, s);
     if (lane == 0) wsum[wi] = s;
     __syncthreads();
     const int blk = wi / (kThreads / 32);
-    uint64_t run = 0;
+    uint32_t run = 0;
     for (int k = blk * (kThreads / 32); k < wi; k++) run += wsum[k];
     for (uint32_t i = 0; i < PER_WARP / 32; i++) {
         const uint32_t wl = wi * PER_WARP + 32 * i + lane;
         const uint64_t b = bm64[wl];
-        const uint64_t c = __popcll(b);
-        uint64_t inc = c;
+        const uint32_t c = __popcll(b);
+        uint32_t inc = c;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            uint64_t u = __shfl_up_sync(0xffffffffu, inc, o);
+            const uint32_t u = __shfl_up_sync(0xffffffffu, inc, o);
             if (lane >= o) inc += u;
         }
         ulonglong2 e;
@@ -361,31 +288,23 @@ uint64_t build_pitable_window(cpx_ctx *ctx, uint64_t w0, uint64_t nwords, cpx_pi
     if (nseg == 0) return 0;
     if (nseg > 0x7FFFFFFFull) fail(CPX_ERANGE, "pi table window too large");
     uint64_t *segtot = ctx->b_segtot.as<uint64_t>(nseg + 1);
-    // sieving primes P[11..] = 37, 41, ...; the kernel stops at p^2 >= segment top
-    const uint32_t nsp_all = (uint32_t)(tb.prm_n > 11 ? tb.prm_n - 11 : 0);
-    const uint32_t ncoop = std::min<uint32_t>(kCoopMax, nsp_all);
-    // four table blocks a CTA when the window is large and a multiple of four blocks
+    // four table blocks a CTA for large windows, one for what is left
     constexpr int kMul = 4;
-    const size_t smem4 = kTabSegWords * 2 * kMul * 4;
-    if (nseg % kMul == 0 && nseg >= (uint64_t)kMul * ctx->sm_count && ctx->smem_optin >= smem4 + 8192) {
-        static std::mutex m;
-        static int done_dev = -1;
-        {
-            std::lock_guard<std::mutex> g(m);
-            if (done_dev != ctx->device) {
-                CPX_CUDA(cudaFuncSetAttribute(k_sieve_table<kMul>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              (int)smem4));
-                done_dev = ctx->device;
-            }
-        }
-        k_sieve_table<kMul><<<(unsigned)(nseg / kMul), kThreads * kMul, smem4, ctx->stream>>>(w0, tb.P + 11, nsp_all,
-                                                                                              ncoop, T, segtot);
-    } else {
-        k_sieve_table<1><<<(unsigned)nseg, kThreads, kTabSegWords * 2 * 4, ctx->stream>>>(w0, tb.P + 11, nsp_all,
-                                                                                         ncoop, T, segtot);
+    uint64_t done = 0;
+    if (nseg >= (uint64_t)kMul * ctx->sm_count) {
+        raise_smem<k_sieve_table<kMul>>(ctx, sieve_block_smem(kThreads * kMul));
+        done = nseg / kMul * kMul;
+        k_sieve_table<kMul><<<(unsigned)(nseg / kMul), kThreads * kMul, sieve_block_smem(kThreads * kMul), ctx->stream>>>(
+            w0, tb.P, (uint32_t)tb.prm_n, T, segtot);
+        CPX_LAUNCH("k_sieve_table");
+        note_launch(ctx);
     }
-    CPX_LAUNCH("k_sieve_table");
-    note_launch(ctx);
+    if (done < nseg) {
+        k_sieve_table<1><<<(unsigned)(nseg - done), kThreads, sieve_block_smem(kThreads), ctx->stream>>>(
+            w0 + done * kTabSegWords, tb.P, (uint32_t)tb.prm_n, T + done * kTabSegWords, segtot + done);
+        CPX_LAUNCH("k_sieve_table");
+        note_launch(ctx);
+    }
     scan_u64(ctx, segtot, nseg);
     k_table_fix<<<(unsigned)((nwords + 255) / 256), 256, 0, ctx->stream>>>(T, nwords, segtot);
     CPX_LAUNCH("k_table_fix");
