@@ -158,20 +158,6 @@ __global__ void __launch_bounds__(512) k_trial_table(cpx_pient *T)
 
 // ------------------------------------------------------ segmented prime sieve
 
-__device__ __forceinline__ uint32_t first_odd_multiple_idx(uint64_t lo, uint64_t hi, uint64_t p,
-                                                            bool from_square)
-{
-    // bit index of the first odd multiple m of p with m >= lo + 1 (and, for
-    // prime sieving, m >= p^2); 0xFFFFFFFF if none below hi.  (lo + 1) mod p
-    // by the reciprocal quotient (p < 2^32), not the 64-bit division routine
-    uint64_t r = (lo + 1) - cpx_udiv_leaf(lo + 1, p) * p;
-    uint64_t m = lo + 1 + (r ? p - r : 0);
-    if ((m & 1) == 0) m += p;
-    if (from_square && m < p * p) m = p * p;
-    if (m >= hi) return 0xFFFFFFFFu;
-    return (uint32_t)((m - lo - 1) >> 1);
-}
-
 // One CTA sieves MUL table blocks of kTabSegWords entries (2^18 odd numbers
 // each) with MUL x 256 threads and writes, per block, its entries (prefix
 // relative to the block) and its total.  A CTA pays the start of every sieving
@@ -438,8 +424,8 @@ uint64_t extract_primes_u64(cpx_ctx *ctx, uint64_t lo, uint64_t hi, uint64_t *d_
 
 // ----------------------------------------------------------- mu / lpf sieve
 
-// odd numbers per CTA: 8 bytes of shared state each for 32-bit words, 12 for 64-bit
-template <class W> struct MuSeg { static constexpr uint32_t N = sizeof(W) == 4 ? 4096 : 2048; };
+// odd numbers per thread of a mu/lpf block, 8 bytes of shared state each
+constexpr uint32_t kMuPer = 16;
 
 // Mitchell's approximation of log2(v), v >= 1, in units of 2^-16: the bit
 // position of the leading one plus the next 16 bits read as a fraction.  It
@@ -464,59 +450,105 @@ __device__ __forceinline__ uint32_t mitchell_log2_q16(uint64_t v)
 // The reference multiplies the prime factors into a word with a
 // compare-and-swap loop (src/sieve/lpf_mu.cu:89-108); the log sum needs none.
 constexpr uint32_t kCofactorQ16 = 91750;  // 1.4 in units of 2^-16
-template <class W>
-__global__ void __launch_bounds__(kThreads) k_mulpf(uint64_t lo0, uint64_t hi_all, const uint32_t *__restrict__ P,
-                                                    uint32_t np, uint32_t nsmall, int8_t *__restrict__ mu,
-                                                    uint32_t *__restrict__ lpf32, uint64_t *__restrict__ lpf64,
-                                                    int32_t *__restrict__ packed)
+
+// floor(lo / p), lod = lo as a double when lo < 2^53 and p >= 2^9 (lo / p below
+// 2^44: the product with the refined reciprocal is within 1 of it)
+__device__ __forceinline__ uint64_t quot_start(uint64_t lo, double lod, bool fast, uint32_t p)
 {
-    constexpr uint32_t kMuSeg = MuSeg<W>::N;
-    __shared__ W s_lpf[kMuSeg];
-    __shared__ uint32_t s_acc[kMuSeg];
-    const uint32_t tid = threadIdx.x;
-    const uint64_t lo = lo0 + (uint64_t)blockIdx.x * 2 * kMuSeg;
-    const uint64_t hi = lo + 2 * kMuSeg;  // exclusive
-    for (uint32_t i = tid; i < kMuSeg; i += kThreads) {
-        s_lpf[i] = (W)~(W)0;
+    if (!fast) return cpx_udiv_leaf(lo, p);
+    const float r0 = cpx_rcp_approx(p);
+    const double rd = __fma_rn((double)r0, __fma_rn(-(double)p, (double)r0, 1.0), (double)r0);
+    uint64_t q = (uint64_t)__double_as_longlong(__dadd_rz(__dmul_rn(lod, rd), 0x1p52)) & 0xFFFFFFFFFFFFFull;
+    const int64_t r = (int64_t)(lo - q * p);
+    if (r < 0) q--;
+    else if (r >= (int64_t)p) q++;
+    return q;
+}
+// the first multiple of p^2 among the n = p k, k = k0, k0 + 2, ... (bit i0 + j p
+// for k0 + 2j): its bit
+__device__ __forceinline__ uint64_t square_start(uint64_t k0, uint64_t i0, uint32_t p)
+{
+    const uint64_t t = cpx_udiv_leaf(k0 + p - 1, p) | 1;  // odd: p t is an odd k
+    return i0 + (((t * p - k0) >> 1) * p);
+}
+
+// One CTA takes kMuPer NT odd numbers with NT threads.  A CTA pays the start of
+// every sieving prime once for all its numbers, and at lo = 1e12 (78 thousand
+// primes) those starts were most of the time when a CTA held 2048 numbers:
+// the CTA is as large as the window and the primes make worth while
+// (mulpf_sieve).  Primes to 31 by all threads, to 2053 a warp each, larger ones
+// a thread each; the multiples of p^2 are found from k = n / p, without a
+// 64-bit division by p^2.  3e7 odd numbers: 0.62 -> 0.24 ms at 0, 2.41 -> 0.40
+// at 1e10, 6.06 -> 1.00 at 1e12 (the 270 MB written take 0.04).
+template <int NT>
+__global__ void __launch_bounds__(NT) k_mulpf(uint64_t lo0, uint64_t hi_all, const uint32_t *__restrict__ P,
+                                              uint32_t np, int8_t *__restrict__ mu, uint32_t *__restrict__ lpf32,
+                                              uint64_t *__restrict__ lpf64, int32_t *__restrict__ packed)
+{
+    constexpr uint32_t N = kMuPer * NT, NWRP = NT / 32;
+    constexpr uint32_t kAll = 11, kWarp = 310;  // P[11] = 37, P[310] = 2063
+    extern __shared__ uint32_t s_lpf[];         // N least prime factors, then N log sums
+    uint32_t *s_acc = s_lpf + N;
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint64_t lo = lo0 + (uint64_t)blockIdx.x * 2 * N;
+    const uint64_t hi = lo + 2 * N;  // exclusive
+    for (uint32_t i = tid; i < N; i += NT) {
+        s_lpf[i] = 0xFFFFFFFFu;
         s_acc[i] = 0;
     }
     __syncthreads();
-    auto square_flags = [&](uint64_t p, uint32_t t0, uint32_t step) {
-        const uint64_t p2 = p * p;
-        if (p2 >= hi) return;
-        uint64_t r = (lo + 1) % p2;
-        uint64_t m = lo + 1 + (r ? p2 - r : 0);
-        if ((m & 1) == 0) m += p2;
-        for (m += (uint64_t)t0 * 2 * p2; m < hi; m += (uint64_t)step * 2 * p2)
-            atomicOr(&s_acc[(m - lo - 1) >> 1], 0x80000000u);
+    const double lod = (double)lo;
+    const bool small = (lo >> 53) == 0;
+    auto mark = [&](uint32_t i, uint32_t p, uint32_t add) {
+        atomicMin(&s_lpf[i], p);
+        atomicAdd(&s_acc[i], add);
     };
-    // primes from P[1] (3) while p^2 < hi; the first nsmall by all threads
-    for (uint32_t k = 1; k < np && k <= nsmall; k++) {
-        const uint64_t p = P[k];
-        if (p * p >= hi) break;
-        uint32_t i0 = first_odd_multiple_idx(lo, hi, p, false);
-        if (i0 == 0xFFFFFFFFu) continue;
+    // primes from P[1] (3) while p^2 < hi; the first by all threads
+    for (uint32_t k = 1; k < np && k < kAll; k++) {
+        const uint32_t p = P[k];
+        if ((uint64_t)p * p >= hi) break;
+        const uint64_t k0 = (cpx_udiv_leaf(lo, p) + 1) | 1, i0 = (k0 * p - lo - 1) >> 1;
         const uint32_t add = mitchell_log2_q16(p) + (1u << 24);
-        for (uint32_t i = i0 + tid * (uint32_t)p; i < kMuSeg; i += kThreads * (uint32_t)p) {
-            atomicMin(&s_lpf[i], (W)p);
-            atomicAdd(&s_acc[i], add);
-        }
-        square_flags(p, tid, kThreads);
+        for (uint32_t i = (uint32_t)i0 + tid * p; i < N; i += NT * p) mark(i, p, add);
+        for (uint32_t i = (uint32_t)square_start(k0, i0, p) + tid * p * p; i < N; i += NT * p * p)
+            atomicOr(&s_acc[i], 0x80000000u);
     }
-    for (uint32_t k = nsmall + 1 + tid; k < np; k += kThreads) {
-        const uint64_t p = P[k];
-        if (p * p >= hi) break;
-        uint32_t i0 = first_odd_multiple_idx(lo, hi, p, false);
-        if (i0 == 0xFFFFFFFFu) continue;
-        const uint32_t add = mitchell_log2_q16(p) + (1u << 24);
-        for (uint32_t i = i0; i < kMuSeg; i += (uint32_t)p) {
-            atomicMin(&s_lpf[i], (W)p);
-            atomicAdd(&s_acc[i], add);
+    // a warp per prime, 32 primes' starts at a time
+    const uint32_t nw = min(np, kWarp);
+    for (uint32_t k0 = kAll + warp; k0 < nw; k0 += 32 * NWRP) {
+        uint32_t lp = 0, li = 0xFFFFFFFFu, ls = 0xFFFFFFFFu;
+        if (k0 + lane * NWRP < nw) {
+            lp = P[k0 + lane * NWRP];
+            if ((uint64_t)lp * lp < hi) {
+                const uint64_t kk = (cpx_udiv_leaf(lo, lp) + 1) | 1, i0 = (kk * lp - lo - 1) >> 1;
+                li = i0 < N ? (uint32_t)i0 : 0xFFFFFFFFu;
+                const uint64_t sq = square_start(kk, i0, lp);
+                ls = sq < N ? (uint32_t)sq : 0xFFFFFFFFu;
+            }
         }
-        square_flags(p, 0, 1);
+        for (uint32_t j = 0; j < 32 && k0 + j * NWRP < nw; j++) {
+            const uint32_t p = __shfl_sync(FULL, lp, j), i0 = __shfl_sync(FULL, li, j), sq = __shfl_sync(FULL, ls, j);
+            if (i0 == 0xFFFFFFFFu) continue;
+            const uint32_t add = mitchell_log2_q16(p) + (1u << 24);
+            for (uint32_t i = i0 + lane * p; i < N; i += 32 * p) mark(i, p, add);
+            if (sq != 0xFFFFFFFFu)
+                for (uint32_t i = sq + lane * p * p; i < N; i += 32 * p * p) atomicOr(&s_acc[i], 0x80000000u);
+        }
+    }
+    // a thread per prime
+    for (uint32_t k = kWarp + tid; k < np; k += NT) {
+        const uint32_t p = P[k];
+        if ((uint64_t)p * p >= hi) break;
+        const uint64_t q = quot_start(lo, lod, small, p);
+        const uint64_t kk = (q + 1) | 1, i0 = (kk * p - lo - 1) >> 1;
+        if (i0 >= N) continue;
+        const uint32_t add = mitchell_log2_q16(p) + (1u << 24);
+        for (uint64_t i = i0; i < N; i += p) mark((uint32_t)i, p, add);
+        const uint64_t sq = square_start(kk, i0, p);
+        if (sq < N) atomicOr(&s_acc[sq], 0x80000000u);  // p^2 > N
     }
     __syncthreads();
-    for (uint32_t i = tid; i < kMuSeg; i += kThreads) {
+    for (uint32_t i = tid; i < N; i += NT) {
         const uint64_t n = lo + 2 * i + 1;
         const uint64_t gi = (n - lo0 - 1) >> 1;
         if (n >= hi_all) break;
@@ -527,7 +559,7 @@ __global__ void __launch_bounds__(kThreads) k_mulpf(uint64_t lo0, uint64_t hi_al
             l = 0xFFFFFFFFull;
         } else {
             const uint32_t a = s_acc[i];
-            l = (s_lpf[i] == (W)~(W)0) ? n : (uint64_t)s_lpf[i];
+            l = s_lpf[i] == 0xFFFFFFFFu ? n : (uint64_t)s_lpf[i];
             if (a & 0x80000000u) m = 0;
             else {
                 const bool cofactor = mitchell_log2_q16(n) > (a & 0xFFFFFFu) + kCofactorQ16;
@@ -541,18 +573,17 @@ __global__ void __launch_bounds__(kThreads) k_mulpf(uint64_t lo0, uint64_t hi_al
         if (packed) packed[gi] = (n == 1) ? 0x7FFFFFFF : (m == 0 ? 0 : m * (int32_t)l);
     }
 }
+constexpr size_t mu_smem(uint32_t nt) { return size_t(nt) * kMuPer * 8; }
 
 // mu of the odd n in [lo, hi) (hi <= 2^32) into a caller buffer with a
 // caller prime list, on a caller stream; launches only, allocates nothing.
 cudaError_t launch_mu_only(cudaStream_t st, uint64_t lo, uint64_t hi, const uint32_t *P, uint32_t np,
                            int8_t *mu)
 {
-    const uint64_t seg = MuSeg<unsigned int>::N;
-    const uint64_t nblk = (hi - lo + 2 * seg - 1) / (2 * seg);
+    const uint64_t span = 2 * kMuPer * kThreads;
+    const uint64_t nblk = (hi - lo + span - 1) / span;
     if (nblk == 0) return cudaSuccess;
-    const uint32_t nsmall = np > 54 ? 53 : (np ? np - 1 : 0);
-    k_mulpf<unsigned int><<<(unsigned)nblk, kThreads, 0, st>>>(lo, hi, P, np, nsmall, mu, nullptr, nullptr,
-                                                                nullptr);
+    k_mulpf<kThreads><<<(unsigned)nblk, kThreads, mu_smem(kThreads), st>>>(lo, hi, P, np, mu, nullptr, nullptr, nullptr);
     return cudaGetLastError();
 }
 
@@ -563,23 +594,22 @@ void mulpf_sieve(cpx_ctx *ctx, uint64_t lo, uint64_t hi, int8_t *mu, uint32_t *l
     if (hi <= lo) return;
     ensure_primes(ctx, cpx_isqrt(hi) + 2);
     const Tables &tb = ctx->tab;
-    const bool w32 = hi <= 0xFFFFFFFFull;
-    const uint64_t seg = w32 ? MuSeg<unsigned int>::N : MuSeg<unsigned long long>::N;
-    const uint64_t nblk = (hi - lo + 2 * seg - 1) / (2 * seg);
-    if (nblk == 0) return;
-    if (nblk > 0x7FFFFFFFull) fail(CPX_ERANGE, "mu/lpf range too large");
-    // primes below 256 go through the all-threads loop
-    uint32_t nsmall = 0;
-    {
-        static const uint32_t small_cnt = 53;  // primes < 256 after 2 ... 251 is the 54th prime
-        nsmall = (uint32_t)std::min<uint64_t>(small_cnt, tb.prm_n ? tb.prm_n - 1 : 0);
-    }
-    if (w32) {
-        k_mulpf<unsigned int><<<(unsigned)nblk, kThreads, 0, ctx->stream>>>(lo, hi, tb.P, (uint32_t)tb.prm_n, nsmall, mu,
-                                                                         lpf32, lpf64, packed);
+    // 16384 odd numbers a CTA when the sieving primes are many and such CTAs fill
+    // the GPU, 8192 (three CTAs an SM) with fewer primes, else 4096
+    const uint64_t n = (hi - lo) / 2, sms = (uint64_t)ctx->sm_count;
+    auto go = [&](auto kern, uint32_t nt) {
+        const uint64_t span = 2ull * kMuPer * nt, nblk = (hi - lo + span - 1) / span;
+        if (nblk > 0x7FFFFFFFull) fail(CPX_ERANGE, "mu/lpf range too large");
+        kern<<<(unsigned)nblk, nt, mu_smem(nt), ctx->stream>>>(lo, hi, tb.P, (uint32_t)tb.prm_n, mu, lpf32, lpf64, packed);
+    };
+    if (hi >> 34 && n >= 2 * sms * kMuPer * 1024) {
+        raise_smem<k_mulpf<1024>>(ctx, mu_smem(1024));
+        go(k_mulpf<1024>, 1024);
+    } else if (n >= 3 * sms * kMuPer * 512) {
+        raise_smem<k_mulpf<512>>(ctx, mu_smem(512));
+        go(k_mulpf<512>, 512);
     } else {
-        k_mulpf<unsigned long long><<<(unsigned)nblk, kThreads, 0, ctx->stream>>>(
-            lo, hi, tb.P, (uint32_t)tb.prm_n, nsmall, mu, lpf32, lpf64, packed);
+        go(k_mulpf<kThreads>, kThreads);
     }
     CPX_LAUNCH("k_mulpf");
     note_launch(ctx);
