@@ -63,7 +63,7 @@ template <class F> static void each_buf(cpx_ctx *ctx, F &&f)
     for (auto &b : ctx->b_scan) f(b);
     for (auto &b : ctx->b_work) f(b);
     for (DevBuf *b : {&ctx->b_segtot, &ctx->b_small, &ctx->b_tmp, &ctx->b_win, &ctx->b_win2, &ctx->b_flush,
-                      &ctx->b_jobs, &ctx->b_jobctl, &ctx->b_snap, &ctx->b_levels, &ctx->b_lvpar})
+                      &ctx->b_jobs, &ctx->b_jobctl, &ctx->b_snap, &ctx->b_levels, &ctx->b_lvpar, &ctx->b_comp})
         f(*b);
 }
 

@@ -96,6 +96,7 @@ struct cpx_ctx {
     cpx::DevBuf b_flush;     // L2 flush buffer (bench only)
     cpx::DevBuf b_jobs, b_jobctl, b_snap;  // offloaded hard-leaf sets and their snapshots
     cpx::DevBuf b_levels;                  // per-level records of a part of a split query
+    cpx::DevBuf b_comp;                    // the m of the composite easy leaves of large queries
     cpx::DevBuf b_lvpar;                   // per-level constants of the lone-query sieve
     unsigned long long *d_acc = nullptr;  // per-query accumulators (grown)
     size_t acc_cap = 0;

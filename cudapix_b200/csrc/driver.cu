@@ -846,7 +846,7 @@ replan:  // again without the batch alpha when its shared sieve would not fit (b
                 if ((mask & TERM_EASY) && pe > pc) n_easy = host_pi(hP, pe) - c;
                 if (mask & TERM_EASY) {
                     // composite easy leaves: levels b with p_b <= iroot4(x), p_b^2 < y and
-                    // max(y/p_b, x/p_b^3) < y
+                    // max(y/p_b, x/p_b^3) < y; a composite m with lpf(m) > p_b exceeds p_b^2
                     const uint64_t nb4 = host_pi(hP, d.r4);
                     for (uint64_t b = c + 1; b <= nb4; b++) {
                         const uint64_t p = hP[b - 1];
@@ -854,6 +854,7 @@ replan:  // again without the batch alpha when its shared sieve would not fit (b
                         const u128 x3 = (x >> 64) ? x / ((u128)p * p * p) : (u128)((uint64_t)x / (p * p * p));
                         uint64_t mlo = d.y / p;
                         if (x3 > (u128)mlo) mlo = x3 >= (u128)d.y ? d.y : (uint64_t)x3;
+                        mlo = std::max<uint64_t>(mlo, p * p);
                         if (mlo >= d.y) continue;
                         const uint64_t mfirst = (mlo + 1) | 1;
                         EasyLvl r;
@@ -933,6 +934,24 @@ replan:  // again without the batch alpha when its shared sieve would not fit (b
             elv.push_back(r);
         }
         n_ecomp += blk_ecomp[k];
+    }
+    // their m as a list when the levels walk many: above 2^17 chunks of 1024 m
+    // (pi(1e17) walks 4 million: 4.6 ms from the table; pi(1e15) 16 thousand: 0.026
+    // ms, where the list's two launches would take as long).  At most 5760 of
+    // 30030 consecutive numbers have no factor up to 13.
+    constexpr uint64_t kCompListChunks = 1u << 17;
+    uint64_t comp_lo = 0, comp_hi = 0, comp_cap = 0;
+    uint32_t comp_pmin = 0;
+    if (n_ecomp >= kCompListChunks) {
+        comp_lo = ~0ull;
+        comp_pmin = 0xFFFFFFFFu;
+        for (const EasyLvl &r : elv) {
+            comp_lo = std::min(comp_lo, r.i_lo);
+            comp_hi = std::max(comp_hi, r.i_hi);
+            comp_pmin = std::min(comp_pmin, r.p);
+        }
+        comp_cap = ((2 * (comp_hi - comp_lo)) / 30030 + 2) * 5760;
+        if (comp_pmin < 13 || comp_cap > 0x3FFFFFFFull) comp_cap = 0;
     }
     if (!lbits_max) lbits_max = 15;
     if (Q == 1 && !shared && (mask & TERM_HARD) && !rq.seg_hi && !rq.hard_levels && !qd[0].direct &&
@@ -1046,6 +1065,13 @@ replan:  // again without the batch alpha when its shared sieve would not fit (b
     pl.elv = d_elv;
     pl.n_elv = (uint32_t)elv.size();
     pl.n_ecomp = n_ecomp;
+    if (comp_cap) {
+        pl.comp_list = ctx->b_comp.as<uint2>(comp_cap + 1);
+        pl.comp_lo = comp_lo;
+        pl.comp_hi = comp_hi;
+        pl.comp_cap = (uint32_t)comp_cap;
+        pl.comp_pmin = comp_pmin;
+    }
     pl.qd = d_qd;
     pl.pre_ord = d_pre;
     pl.pre_p2 = d_pre + (Q + 1);

@@ -557,9 +557,18 @@ __global__ void __launch_bounds__(kThreads) k_easy(const QD *__restrict__ qd, ui
 }
 
 // Composite easy leaves: p_b <= min(iroot4(x), sqrt y), m composite with
-// lpf(m) > p_b, mu(m) != 0, max(y/p_b, x/p_b^3) < m <= y; value
-// -mu(m) (pi(x/(p_b m)) - b + 2).  Work = (level record, chunk of 1024 odd m);
-// a warp walks its chunk 128 m at a time, one 16-byte load of packed mu*lpf per lane.
+// lpf(m) > p_b, mu(m) != 0, max(y/p_b, x/p_b^3, p_b^2) < m <= y; value
+// -mu(m) (pi(x/(p_b m)) - b + 2).
+//
+// The leaf's pi(u), u = xp / m: u < p_b^2, so below 2^40 for p_b < 2^20
+template <class XT> __device__ __forceinline__ int64_t comp_pi(const cpx_pient *__restrict__ T, XT xp, double xpd, bool f40, uint32_t m)
+{
+    const uint64_t u = f40 ? cpx_quot40((uint64_t)xp, xpd, m) : (uint64_t)cpx_qdiv(xp, (uint64_t)m);
+    return (int64_t)cpx_pi_ge2(T, u);
+}
+
+// From the packed mu*lpf table: work = (level record, chunk of 1024 odd m); a
+// warp walks its chunk 128 m at a time, one 16-byte load per lane.
 template <class XT>
 __global__ void __launch_bounds__(kThreads) k_easy_comp(const QD *__restrict__ qd, const EasyLvl *__restrict__ lv,
                                                         uint32_t nlv, uint64_t total,
@@ -580,6 +589,8 @@ __global__ void __launch_bounds__(kThreads) k_easy_comp(const QD *__restrict__ q
         const EasyLvl r = lv[lo];
         const QD &d = qd[r.q];
         const XT xp = cpx_qdiv(xload<XT>(d), r.p);
+        const double xpd = (double)(uint64_t)xp;
+        const bool f40 = xp < ((XT)1 << 53) && r.p < (1u << 20);
         const uint64_t base = r.i_base + (unit - r.unit0) * 1024;  // multiple of 4
         int64_t s = 0;
         for (int it = 0; it < 8; it++) {
@@ -592,13 +603,85 @@ __global__ void __launch_bounds__(kThreads) k_easy_comp(const QD *__restrict__ q
                 const uint64_t i = i0 + k;
                 if (i < r.i_lo || i >= r.i_hi) continue;
                 const int32_t v = vals[k];
-                const uint64_t m = 2 * i + 1;
+                const uint32_t m = (uint32_t)(2 * i + 1);
                 const uint32_t av = (uint32_t)(v > 0 ? v : -v);
-                if (v == 0 || av <= r.p || (uint64_t)av >= m) continue;  // mu = 0, lpf <= p, or m prime
-                const uint64_t uu = (uint64_t)cpx_qdiv(xp, m);
-                const int64_t val = (int64_t)cpx_pi_dev(T, uu) - (int64_t)r.b + 2;
+                if (v == 0 || av <= r.p || av >= m) continue;  // mu = 0, lpf <= p, or m prime
+                const int64_t val = comp_pi<XT>(T, xp, xpd, f40, m) - (int64_t)r.b + 2;
                 s += (v > 0) ? -val : val;
             }
+        }
+        LaneAcc a;
+        a.q = r.q;
+        a.v = s;
+        warp_flush(a, acc, ACC_EASY);
+    }
+}
+
+// From a list: the levels of a large query all walk nearly the same m, of which
+// few are composite with a least factor above the levels' smallest prime pmin
+// (pi(1e17): 7e9 m over 630 levels for 1.6e7 leaves).  k_comp_list writes those
+// down once, {m | (mu(m) = -1) << 31, lpf(m)} in no order, and each level goes
+// through the list: pi(1e17) 4.59 -> 0.24 ms, pi(1.9e19) 18.8 -> 0.44.  cap entries always suffice (the host's bound).
+__global__ void __launch_bounds__(kThreads) k_comp_list(const int32_t *__restrict__ MU, uint64_t i_lo, uint64_t i_hi,
+                                                        uint32_t pmin, uint32_t cap, uint2 *__restrict__ list,
+                                                        unsigned int *__restrict__ count)
+{
+    const uint64_t i0 = 4 * ((i_lo >> 2) + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x);
+    const uint32_t lane = threadIdx.x & 31;
+    uint2 e[4];
+    uint32_t n = 0;
+    if (i0 < i_hi) {
+        const int4 v4 = __ldg(reinterpret_cast<const int4 *>(MU) + (i0 >> 2));
+        const int32_t vals[4] = {v4.x, v4.y, v4.z, v4.w};
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const uint64_t i = i0 + k;
+            const int32_t v = vals[k];
+            const uint32_t m = (uint32_t)(2 * i + 1), av = (uint32_t)(v > 0 ? v : -v);
+            if (i < i_lo || i >= i_hi || v == 0 || av <= pmin || av >= m) continue;
+            e[n++] = make_uint2(m | (v < 0 ? 0x80000000u : 0u), av);
+        }
+    }
+    uint32_t inc = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(FULL, inc, o);
+        if (lane >= (uint32_t)o) inc += t;
+    }
+    const uint32_t tot = __shfl_sync(FULL, inc, 31);
+    if (!tot) return;
+    uint32_t at = 0;
+    if (lane == 0) at = atomicAdd(count, tot);
+    at = __shfl_sync(FULL, at, 0) + inc - n;
+    for (uint32_t k = 0; k < n; k++)
+        if (at + k < cap) list[at + k] = e[k];
+}
+
+// work = (level record, chunk of 1024 list entries), a warp each
+template <class XT>
+__global__ void __launch_bounds__(kThreads) k_easy_comp_list(const QD *__restrict__ qd, const EasyLvl *__restrict__ lv,
+                                                             uint32_t nlv, const uint2 *__restrict__ list,
+                                                             const unsigned int *__restrict__ count, uint32_t cap,
+                                                             const cpx_pient *__restrict__ T,
+                                                             unsigned long long *__restrict__ acc)
+{
+    const uint32_t lane = threadIdx.x & 31, n = min(*count, cap), nch = (n + 1023) / 1024;
+    const uint64_t gw = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    for (uint64_t unit = gw; unit < (uint64_t)nlv * nch; unit += nw) {
+        const EasyLvl r = lv[unit / nch];
+        const XT xp = cpx_qdiv(xload<XT>(qd[r.q]), r.p);
+        const double xpd = (double)(uint64_t)xp;
+        const bool f40 = xp < ((XT)1 << 53) && r.p < (1u << 20);
+        const uint32_t m_lo = (uint32_t)(2 * r.i_lo + 1), m_hi = (uint32_t)(2 * r.i_hi);  // m in [m_lo, m_hi)
+        const uint32_t k0 = (uint32_t)(unit % nch) * 1024, k1 = min(n, k0 + 1024);
+        int64_t s = 0;
+        for (uint32_t k = k0 + lane; k < k1; k += 32) {
+            const uint2 e = __ldg(list + k);
+            const uint32_t m = e.x & 0x7FFFFFFFu;
+            if (e.y <= r.p || m < m_lo || m >= m_hi) continue;
+            const int64_t val = comp_pi<XT>(T, xp, xpd, f40, m) - (int64_t)r.b + 2;
+            s += (e.x >> 31) ? val : -val;
         }
         LaneAcc a;
         a.q = r.q;
@@ -745,7 +828,23 @@ void launch_easy_comp(cpx_ctx *ctx, const Plan &pl)
     const unsigned grid = (unsigned)std::max<uint64_t>(
         1, std::min<uint64_t>((pl.n_ecomp + (kThreads / 32) - 1) / (kThreads / 32), (uint64_t)ctx->sm_count * 16));
     KSpan ks(ctx, "k_easy_comp");
-    if (pl.wide)
+    if (pl.comp_list) {
+        uint2 *list = static_cast<uint2 *>(pl.comp_list);
+        unsigned int *count = reinterpret_cast<unsigned int *>(list + pl.comp_cap);
+        CPX_CUDA(cudaMemsetAsync(count, 0, sizeof(unsigned int), ctx->stream));
+        const uint64_t groups = ((pl.comp_hi + 3) >> 2) - (pl.comp_lo >> 2);
+        k_comp_list<<<(unsigned)((groups + kThreads - 1) / kThreads), kThreads, 0, ctx->stream>>>(
+            ctx->tab.MU, pl.comp_lo, pl.comp_hi, pl.comp_pmin, pl.comp_cap, list, count);
+        CPX_LAUNCH("k_comp_list");
+        note_launch(ctx);
+        const unsigned g = (unsigned)ctx->sm_count * 8;
+        if (pl.wide)
+            k_easy_comp_list<u128><<<g, kThreads, 0, ctx->stream>>>(pl.qd, pl.elv, pl.n_elv, list, count, pl.comp_cap,
+                                                                    ctx->tab.T, pl.acc);
+        else
+            k_easy_comp_list<uint64_t><<<g, kThreads, 0, ctx->stream>>>(pl.qd, pl.elv, pl.n_elv, list, count,
+                                                                        pl.comp_cap, ctx->tab.T, pl.acc);
+    } else if (pl.wide)
         k_easy_comp<u128><<<grid, kThreads, 0, ctx->stream>>>(pl.qd, pl.elv, pl.n_elv, pl.n_ecomp, ctx->tab.MU,
                                                               ctx->tab.T, pl.acc);
     else

@@ -107,6 +107,11 @@ struct Plan {
     const EasyLvl *elv = nullptr;
     uint32_t n_elv = 0;
     uint64_t n_ecomp = 0;
+    // their m of all levels at once (odd indices [comp_lo, comp_hi), lpf above
+    // comp_pmin) as a list of comp_cap entries and a counter; null: from the table
+    void *comp_list = nullptr;
+    uint64_t comp_lo = 0, comp_hi = 0;
+    uint32_t comp_cap = 0, comp_pmin = 0;
     bool p2_primes = false;        // P2 units are the primes of (y, sqrt x] (k_p2_primes), else pi-table entries
     uint64_t *easy_off = nullptr;  // n_easy + 1 chunk offsets of the easy leaves
     void *easy_rec = nullptr;      // n_easy unit plans (EasyRec, 64 B each), or null: k_easy plans itself
