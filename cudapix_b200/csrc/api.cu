@@ -61,6 +61,7 @@ namespace cpx {
 template <class F> static void each_buf(cpx_ctx *ctx, F &&f)
 {
     for (auto &b : ctx->b_scan) f(b);
+    for (auto &b : ctx->b_scan2) f(b);
     for (auto &b : ctx->b_work) f(b);
     for (DevBuf *b : {&ctx->b_segtot, &ctx->b_small, &ctx->b_tmp, &ctx->b_win, &ctx->b_win2, &ctx->b_flush,
                       &ctx->b_jobs, &ctx->b_jobctl, &ctx->b_snap, &ctx->b_levels, &ctx->b_lvpar, &ctx->b_comp})
@@ -95,6 +96,7 @@ void release_context(cpx_ctx *ctx)
     std::lock_guard<std::recursive_mutex> lk(ctx->mu);
     DeviceGuard dg(ctx->device);
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
+    if (ctx->side) cudaStreamSynchronize(ctx->side);
     Tables &tb = ctx->tab;
     if (!ctx->tables_borrowed) {
         if (tb.T) cudaFree(tb.T);
@@ -116,6 +118,12 @@ void release_context(cpx_ctx *ctx)
         if (ev) cudaEventDestroy(ev);
         ev = nullptr;
     }
+    for (cudaEvent_t *ev : {&ctx->ev_fork, &ctx->ev_join}) {
+        if (*ev) cudaEventDestroy(*ev);
+        *ev = nullptr;
+    }
+    if (ctx->side) cudaStreamDestroy(ctx->side);
+    ctx->side = nullptr;
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     ctx->stream = nullptr;
 }

@@ -87,6 +87,11 @@ struct cpx_ctx {
     cudaStream_t stream = nullptr;
     cpx::Tables tab;
     cpx::DevBuf b_scan[3];   // block sums of the three scan levels
+    cpx::DevBuf b_scan2[3];  // the same for scans on the side stream
+    // the other terms of a query beside its hard leaves (driver.cu), ordered
+    // against the context's stream by the two events
+    cudaStream_t side = nullptr;
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     cpx::DevBuf b_segtot;    // per-segment totals of a table build
     cpx::DevBuf b_small;     // a few words for pi lookups and totals
     cpx::DevBuf b_tmp;       // bootstrap table, wheel flags
@@ -162,6 +167,28 @@ void ensure_wheel(cpx_ctx *ctx, uint32_t c);
 // the window start, i.e. counts odd primes >= 128*w0), using the resident
 // primes (must cover sqrt of the window top).  Returns total odd primes.
 uint64_t build_pitable_window(cpx_ctx *ctx, uint64_t w0, uint64_t nwords, cpx_pient *T);
+
+// creates the side stream and its events on first use (not while capturing)
+void ensure_side(cpx_ctx *ctx);
+// While this lives, work put on the context's side stream (StreamScope) runs
+// beside that on its own stream, after the point where ev_fork was recorded
+// there; at the end (also when a launch throws) the own stream waits for it.
+struct SideFork {
+    cpx_ctx *c;
+    SideFork(cpx_ctx *ctx, bool on);
+    ~SideFork();
+    SideFork(const SideFork &) = delete;
+    SideFork &operator=(const SideFork &) = delete;
+};
+// launches go to stream s while this lives
+struct StreamScope {
+    cpx_ctx *c;
+    cudaStream_t prev;
+    StreamScope(cpx_ctx *ctx, cudaStream_t s) : c(ctx), prev(ctx->stream) { c->stream = s; }
+    ~StreamScope() { c->stream = prev; }
+    StreamScope(const StreamScope &) = delete;
+    StreamScope &operator=(const StreamScope &) = delete;
+};
 
 // exclusive scan of n uint64 values in place (device)
 void scan_u64(cpx_ctx *ctx, uint64_t *d, uint64_t n);

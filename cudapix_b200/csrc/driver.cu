@@ -351,14 +351,17 @@ static double leaf_estimate(const QD &d, const std::vector<uint32_t> &hP, uint32
     return sum;
 }
 
-// The units before each of the first segments whose leaves take more time than
-// the rest of a unit (k_hard): such a segment's leaves are split over several
-// units, each of which sieves the segment again.  A unit costs each of its
-// warps about 600 issue slots for each of the first 64 levels and 80 for each
-// of the others, a leaf kLeafSlots.  A unit should
-// not take more than about half of a resident CTA's share of the whole query
-// either (the first segments start first, and the rest fills in behind them).
-constexpr double kLeafSlots = 5.0;
+// The units before each of the first segments whose leaves are split over
+// several units (k_hard), each of which sieves the segment again.  A unit costs
+// each of its warps about 600 issue slots for each of the first 64 levels and
+// 80 for each of the others, a leaf about kLeafSlots.  Leaves worth kUnitShare
+// of a resident CTA's part of the whole query are split, so that no unit
+// outlasts the launch, and no finer than the unit's other work is worth (a
+// quarter of it while the units do not fill the GPU).  On a B200, ms of
+// pi(1e15) and pi(1e17) with kUnitShare 0.15 / 0.3 / 0.6 / 0.9: 2.53 / 2.44 /
+// 2.36 / 2.39 and 34.1 / 32.1 / 30.9 / 30.4; pi(1e12) with kUnitFixed 1 / 0.5 /
+// 0.25: 0.285 / 0.227 / 0.210.
+constexpr double kLeafSlots = 6.0, kUnitShare = 0.6, kUnitFixed = 0.25;
 static void dense_units(const QD &d, const std::vector<uint32_t> &hP, uint32_t c, uint32_t threads, uint32_t ctas,
                         std::vector<uint32_t> &base)
 {
@@ -398,12 +401,13 @@ static void dense_units(const QD &d, const std::vector<uint32_t> &hP, uint32_t c
         pts.push_back(t);
         k += n;
     }
-    const double share = 0.5 * total / ctas;
+    const double share = kUnitShare * total / ctas;
+    const double fixed_part = std::min(1.0, std::max(kUnitFixed, (double)d.nseg / ctas));
     std::vector<uint32_t> parts;
     size_t last = 0;  // segments up to the last one with several units
     for (size_t j = 0; j < pts.size() && pts[j].seg < (1u << 16); j++) {
         const uint64_t end = j + 1 < pts.size() ? pts[j + 1].seg : d.nseg;
-        const double unit = std::max(pts[j].fixed, share);
+        const double unit = std::max(fixed_part * pts[j].fixed, share);
         const uint32_t n = unit > 0 ? (uint32_t)std::min(64.0, std::ceil(pts[j].leaf / unit)) : 1;
         if (n >= 2) last = end;
         parts.resize(end, std::max(n, 1u));
@@ -818,6 +822,8 @@ replan:  // again without the batch alpha when its shared sieve would not fit (b
              *p_seg = p_easy + (Q + 1), *p_comb = p_seg + (Q + 1);
     std::vector<uint64_t> q_ent(Q, 0), q_rows(Q, 0);
     std::vector<std::vector<uint32_t>> q_dense(shared || !(mask & TERM_HARD) ? 0 : Q);
+    // CTAs of the lone-query sieve the GPU holds at once (registers: 64 a thread)
+    const uint32_t resident = (uint32_t)ctx->sm_count * std::max<uint32_t>(1, std::min<uint32_t>(1024 / threads, 4));
     const size_t nblk = (Q + kPlanBlock - 1) / kPlanBlock;
     std::vector<std::vector<EasyLvl>> blk_elv(nblk);
     std::vector<uint64_t> blk_ecomp(nblk, 0);
@@ -885,7 +891,7 @@ replan:  // again without the batch alpha when its shared sieve would not fit (b
                     n_comb = d.nb - c;
                     // units: the segments, the dense ones several times
                     std::vector<uint32_t> &base = q_dense[i];
-                    dense_units(d, hP, c, threads, (uint32_t)ctx->sm_count * 2, base);
+                    dense_units(d, hP, c, threads, resident, base);
                     uint64_t extra = 0;
                     for (size_t k = 0; k + 1 < base.size(); k++) {
                         const uint64_t more = base[k + 1] - base[k] - 1, lo = (d.seg0 + k) * span, hi = lo + span;
@@ -1188,22 +1194,36 @@ replan:  // again without the batch alpha when its shared sieve would not fit (b
     CPX_CUDA(cudaMemsetAsync(d_acc, 0, acc_words * 8 + 8, ctx->stream));  // and the unit counter
 
     // ---- kernels
+    // One sieve per query leaves most of the GPU idle for small x (pi(1e8): two
+    // CTAs) and has a tail for large, so the other terms run beside it on the
+    // side stream, from the moment it starts (started earlier, the easy leaves
+    // take the SMs of its densest segments: Gourdon's terms of 1e15 3.4 against
+    // 3.1 ms).  The batch-shared sieve fills every SM and its terms follow one
+    // another, as they do while kernels are timed.
+    ctx->span_on = ctx->timing && !rq.graph;
+    const bool beside = (mask & ~(unsigned)TERM_HARD) && !pl.shared && pl.n_seg && !ctx->span_on;
+    if (beside) ensure_side(ctx);
+    pl.fork = beside;
     auto launch_all = [&] {
-        if (mask & TERM_ORD) launch_ordinary(ctx, pl);
-        if (mask & TERM_P2) launch_p2(ctx, pl);
-        if (mask & TERM_TRIV) launch_trivial(ctx, pl);
-        if (mask & TERM_EASY) {
-            launch_easy(ctx, pl);
-            launch_easy_comp(ctx, pl);
+        {
+            if (beside) launch_hard(ctx, pl);
+            SideFork fork(ctx, beside);
+            StreamScope on(ctx, beside ? ctx->side : ctx->stream);
+            if (mask & TERM_ORD) launch_ordinary(ctx, pl);
+            if (mask & TERM_P2) launch_p2(ctx, pl);
+            if (mask & TERM_TRIV) launch_trivial(ctx, pl);
+            if (mask & TERM_EASY) {
+                launch_easy(ctx, pl);
+                launch_easy_comp(ctx, pl);
+            }
         }
-        if (mask & TERM_HARD) {
+        if ((mask & TERM_HARD) && !beside) {
             if (pl.shared) launch_hard_shared(ctx, pl);
             else launch_hard(ctx, pl);
         }
         if (!any_p2win) launch_finalize(ctx, pl, d_out, mask == TERM_PI);
     };
     ctx->n_span = 0;
-    ctx->span_on = ctx->timing && !rq.graph;
     if (ctx->timing) CPX_CUDA(cudaEventRecord(ctx->ev_b0, ctx->stream));
     if (rq.graph && !any_p2win) launch_as_graph(ctx, launch_all);
     else launch_all();

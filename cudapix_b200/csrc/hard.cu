@@ -10,7 +10,7 @@
 // One CTA owns one unit: a segment of 2^lbits odd numbers n = lo + 2i + 1 and
 // all of its leaves, or every nparts-th 32 table entries of their candidates
 // where the segment holds more leaves than the rest of its work (the early
-// segments: their number falls as 1/u^2).  Each warp owns a contiguous
+// segments: their number falls as 1/u^2; dense_units in driver.cu).  Each warp owns a contiguous
 // sub-segment as a bitmap in shared memory with one 8-bit survivor counter per
 // 16-byte chunk (128 numbers), and walks the levels b = c+1 .. B(seg) on its
 // own, synchronising only inside the warp, 32 levels (a block) at a time: one
@@ -155,7 +155,7 @@ __global__ void __launch_bounds__(512, 2) k_hard(const QD *__restrict__ qd, uint
     const uint32_t c0 = CPT * tid;  // first owned chunk (of the segment)
     const uint32_t cw0 = c0 - CPT * 32 * warp;  // first owned chunk of the sub-segment
     // ---- pre-sieve with p_2 .. p_c; chunk counters
-    const uint32_t cnt0 = presieve(bm, cnt8, P, c, lo, c0, CPT, s);
+    const uint32_t cnt0 = presieve(bm, cnt8, c, lo, c0, CPT, s);
     uint32_t tot = __reduce_add_sync(FULL, cnt0);  // survivors of this warp's sub-segment
     __syncwarp();
 
@@ -768,6 +768,7 @@ template <class XT> static void hard_go(cpx_ctx *ctx, const Plan &pl)
     scan_u64(ctx, pl.seg_off, pl.n_seg);
     const size_t smem = levels_smem(pl.lbits_max, pl.hard_threads);
     if (pl.time_hard) CPX_CUDA(cudaEventRecord(ctx->ev_hard0, ctx->stream));
+    if (pl.fork) CPX_CUDA(cudaEventRecord(ctx->ev_fork, ctx->stream));
     {
         KSpan ks(ctx, "k_hard");
         k_hard<XT><<<(unsigned)pl.n_seg, pl.hard_threads, smem, ctx->stream>>>(

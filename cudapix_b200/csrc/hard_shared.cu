@@ -81,7 +81,7 @@ __global__ void __launch_bounds__(1024, 1) k_sieve_counts(uint64_t nseg, uint32_
     uint32_t *bm = reinterpret_cast<uint32_t *>(smem4);
     uint8_t *cnt8 = reinterpret_cast<uint8_t *>(smem4) + L / 8;
     const uint32_t c0 = CPT * tid, cw0 = c0 - CPT * 32 * warp;
-    uint32_t tot = __reduce_add_sync(FULL, presieve(bm, cnt8, P, c, lo, c0, CPT, s));
+    uint32_t tot = __reduce_add_sync(FULL, presieve(bm, cnt8, c, lo, c0, CPT, s));
     __syncwarp();
     const uint64_t w = seg * NW + warp;
     for (uint32_t gb = c + 1; gb <= B; gb += 32) {
@@ -361,7 +361,7 @@ template <class XT> __device__ __forceinline__ void hard_shared_unit(uint64_t un
     __syncthreads();
 
     const uint32_t c0 = CPT * tid, cw0 = c0 - CPT * 32 * warp;
-    presieve(bm, cnt8, P, c, lo, c0, CPT, s);
+    presieve(bm, cnt8, c, lo, c0, CPT, s);
     __syncwarp();
     const uint64_t w = seg * NW + warp;
     auto sub_count = [&](uint64_t uu) -> uint32_t { return sub_survivors_pre(uu, lo_w, wl, pre16, bm, CPT, s, warp); };

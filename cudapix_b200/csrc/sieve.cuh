@@ -64,38 +64,51 @@ __host__ __device__ __forceinline__ size_t snap_stride(uint32_t lbits_sub)
 constexpr uint32_t kLeafBuf = 256;
 
 // Pre-sieve of one lane's chunks [c0, c0 + CPT) of the segment starting at lo
-// with p_2 .. p_c (residue masks per 32-bit word); writes the bitmap and the
-// chunk counters and returns the lane's survivors.  Runs once per segment, so
-// it is kept out of line (instruction-cache footprint of the level loop).
-static __device__ __noinline__ uint32_t presieve(uint32_t *bm, uint8_t *cnt8, const uint32_t *__restrict__ P, uint32_t c,
-                                          uint64_t lo, uint32_t c0, uint32_t CPT, int s)
+// with p_2 .. p_c, c <= 8 (residue masks per 32-bit word, the primes constants
+// of the code); writes the bitmap and the chunk counters and returns the lane's
+// survivors.  Runs once per segment, so it is kept out of line
+// (instruction-cache footprint of the level loop).
+template <uint32_t I> struct PreP { static constexpr uint32_t p = I == 0 ? 3 : I == 1 ? 5 : I == 2 ? 7 : I == 3 ? 11 : I == 4 ? 13 : I == 5 ? 17 : 19; };
+constexpr uint32_t every_pth_bit_c(uint32_t p)
 {
-    uint32_t pr[8], rr[8], st[8], Mp[8];
-    const uint32_t np = c - 1;
-    const uint32_t w0 = 4 * c0;
-#pragma unroll
-    for (uint32_t i = 0; i < 8; i++) {
-        if (i < np) {
-            pr[i] = P[i + 1];
-            rr[i] = (uint32_t)(((lo + 1) % pr[i] + (64ull * w0) % pr[i]) % pr[i]);
-            st[i] = 64u % pr[i];
-            Mp[i] = every_pth_bit(pr[i]);
-        }
-    }
+    uint32_t m = 0;
+    for (uint32_t k = 0; k < 32; k += p) m |= 1u << k;
+    return m;
+}
+template <uint32_t I> __device__ __forceinline__ uint32_t pre_residue(uint64_t lo, uint32_t w0)
+{
+    constexpr uint32_t p = PreP<I>::p;
+    return ((uint32_t)((lo + 1) % p) + (64u % p) * (w0 % p)) % p;
+}
+// the multiples of PreP<I> in a word whose first number is r mod p; steps r to the next word
+template <uint32_t I> __device__ __forceinline__ uint32_t pre_mask(uint32_t &r)
+{
+    constexpr uint32_t p = PreP<I>::p, Mp = every_pth_bit_c(p), st = 64u % p;
+    const uint32_t m = mult_mask(r, p, Mp);
+    r += st;
+    if (r >= p) r -= p;
+    return m;
+}
+static __device__ __noinline__ uint32_t presieve(uint32_t *bm, uint8_t *cnt8, uint32_t c, uint64_t lo, uint32_t c0,
+                                                 uint32_t CPT, int s)
+{
+    const uint32_t np = c - 1, w0 = 4 * c0;
+    uint32_t r0 = pre_residue<0>(lo, w0), r1 = pre_residue<1>(lo, w0), r2 = pre_residue<2>(lo, w0),
+             r3 = pre_residue<3>(lo, w0), r4 = pre_residue<4>(lo, w0), r5 = pre_residue<5>(lo, w0),
+             r6 = pre_residue<6>(lo, w0);
     uint32_t cnt0 = 0;
     for (uint32_t j = 0; j < CPT; j++) {
         uint32_t wv[4];
 #pragma unroll
         for (int k = 0; k < 4; k++) {
             uint32_t m = 0;
-#pragma unroll
-            for (uint32_t i = 0; i < 8; i++) {
-                if (i < np) {
-                    m |= mult_mask(rr[i], pr[i], Mp[i]);
-                    rr[i] += st[i];
-                    if (rr[i] >= pr[i]) rr[i] -= pr[i];
-                }
-            }
+            if (np > 0) m |= pre_mask<0>(r0);
+            if (np > 1) m |= pre_mask<1>(r1);
+            if (np > 2) m |= pre_mask<2>(r2);
+            if (np > 3) m |= pre_mask<3>(r3);
+            if (np > 4) m |= pre_mask<4>(r4);
+            if (np > 5) m |= pre_mask<5>(r5);
+            if (np > 6) m |= pre_mask<6>(r6);
             wv[k] = ~m;
         }
         const uint32_t cc = __popc(wv[0]) + __popc(wv[1]) + __popc(wv[2]) + __popc(wv[3]);

@@ -56,6 +56,28 @@ void DevBuf::release()
     bytes = 0;
 }
 
+void ensure_side(cpx_ctx *ctx)
+{
+    if (ctx->side) return;
+    for (cudaEvent_t *ev : {&ctx->ev_fork, &ctx->ev_join})
+        if (!*ev) CPX_CUDA(cudaEventCreateWithFlags(ev, cudaEventDisableTiming));
+    CPX_CUDA(cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking));
+}
+
+SideFork::SideFork(cpx_ctx *ctx, bool on) : c(nullptr)
+{
+    if (!on) return;
+    CPX_CUDA(cudaStreamWaitEvent(ctx->side, ctx->ev_fork, 0));
+    c = ctx;
+}
+SideFork::~SideFork()
+{
+    if (!c) return;
+    // (an error here shows again at the batch's synchronisation)
+    cudaEventRecord(c->ev_join, c->side);
+    cudaStreamWaitEvent(c->stream, c->ev_join, 0);
+}
+
 // ------------------------------------------------------------------- scans
 
 constexpr int kScanItems = 4;  // per thread
@@ -102,7 +124,7 @@ static void scan_u64_rec(cpx_ctx *ctx, uint64_t *d, uint64_t n, int depth)
     if (n == 0) return;
     uint64_t nb = (n + kScanBlock - 1) / kScanBlock;
     if (depth > 2) fail(CPX_ERANGE, "scan too large");
-    uint64_t *sums = ctx->b_scan[depth].as<uint64_t>(nb + 1);
+    uint64_t *sums = (ctx->stream == ctx->side ? ctx->b_scan2 : ctx->b_scan)[depth].as<uint64_t>(nb + 1);
     k_scan_block<<<(unsigned)nb, kThreads, 0, ctx->stream>>>(d, n, sums);
     CPX_LAUNCH("k_scan_block");
     note_launch(ctx);
@@ -121,6 +143,7 @@ void scan_reserve(cpx_ctx *ctx, uint64_t n)
     for (int depth = 0; depth < 3 && n > 0; depth++) {
         const uint64_t nb = (n + kScanBlock - 1) / kScanBlock;
         ctx->b_scan[depth].as<uint64_t>(nb + 1);
+        ctx->b_scan2[depth].as<uint64_t>(nb + 1);
         if (nb <= 1) break;
         n = nb;
     }

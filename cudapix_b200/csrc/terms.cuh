@@ -83,6 +83,7 @@ struct Plan {
     uint32_t c = 6;
     bool wide = false;  // 128-bit kernels (some x >= 2^64, or requested)
     bool time_hard = false;  // CUDA events around the hard-leaf kernels
+    bool fork = false;       // ev_fork is recorded just before the lone-query sieve
     uint32_t hard_threads = 256;
     uint32_t lbits_max = 18;
     // device work arrays
