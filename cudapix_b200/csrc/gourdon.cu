@@ -23,84 +23,61 @@
 //
 // B, C, D and Phi0 come from the Deleglise-Rivat kernels (k_p2 plus a closed
 // form, k_easy limited to p <= x* with k_easy_comp, the hard-leaf sieve,
-// k_ordinary).  A is k_gourdon_A: warps take the p of (x*, cbrt x] one at a
-// time from a device counter (largest q range first), gather the primes q of
-// a run of pi-table entries into shared memory and answer them 32 at a time,
-// one quotient and one table lookup per pair.  The Sigma sums and the trivial
-// leaves of C are k_gourdon_sums, one thread per p.  x < 2^64, as the
-// reference's GourdonVariant64.
+// k_ordinary).  A is k_gourdon_A: CTAs take the p of (x*, cbrt x] one at a time
+// from a device counter (largest q range first) and read its primes q from the
+// prime list, one quotient and one table lookup per pair.  The Sigma sums and
+// the trivial leaves of C are k_gourdon_sums, one thread per p.  x < 2^64, as
+// the reference's GourdonVariant64.
 #include "driver.h"
-#include "sieve.cuh"
+#include "kern_common.cuh"
 
 namespace cpx {
 
 namespace {
 
 enum { G_A = 0, G_S4, G_S5, G_S6, G_CT, G_N };  // 128-bit device sums
-constexpr uint32_t kGABuf = 256;                // gathered q per warp
 
-// A over the primes p = P[i], i in [i0, i1): per p the q in (p, sqrt(x/p)]
+// A over the primes p = P[i], i in [i0, i1): per p the primes q in (p, sqrt(x/p)],
+// P[i + 1] on, read from the prime list (which reaches sqrt(x / P[i0])).  A CTA
+// takes one p at a time, four leaves a thread a step so that their table gathers
+// overlap: with a warp per p the first p's q (35 thousand of 1e15's) outlasted
+// the launch.  u = x/(pq) < sqrt x < 2^32 and x/p < 2^48 for p > x^(1/4), so
+// every quotient is cpx_quot40's.  x = 1e15: 0.83 ms a warp per p
+// gathering its q from the pi table, 0.20 so.
 __global__ void __launch_bounds__(256) k_gourdon_A(uint64_t x, uint64_t y, const uint32_t *__restrict__ P,
                                                    uint32_t i0, uint32_t i1, const cpx_pient *__restrict__ T,
                                                    unsigned int *__restrict__ next, unsigned long long *__restrict__ acc)
 {
-    const uint32_t lane = threadIdx.x & 31;
-    __shared__ uint32_t s_q[256 / 32][kGABuf];
-    uint32_t *qbuf = s_q[threadIdx.x >> 5];
+    const uint32_t tid = threadIdx.x;
+    __shared__ uint32_t s_k;
     u128 sum = 0;
     for (;;) {
-        uint32_t k = 0;
-        if (lane == 0) k = atomicAdd(next, 1u);
-        k = __shfl_sync(FULL, k, 0);
+        __syncthreads();
+        if (tid == 0) s_k = atomicAdd(next, 1u);
+        __syncthreads();
+        const uint32_t k = s_k;
         if (k >= i1 - i0) break;
         const uint64_t p = __ldg(P + i0 + k);
         const uint64_t xp = cpx_udiv_leaf(x, p);
         const uint64_t qhi = cpx_isqrt((u128)xp);
-        if (qhi <= p) continue;  // uniform over the warp
-        const uint64_t w_beg = p >> 7, w_end = ((qhi - 1) >> 7) + 1;
+        if (qhi <= p) continue;  // uniform over the CTA
+        const uint32_t *Pq = P + i0 + k + 1;
+        const uint32_t nq = (uint32_t)cpx_pi_ge2(T, qhi) - (i0 + k + 1);  // p = P[i0 + k] is the (i0 + k + 1)-th prime
+        const double xpd = (double)xp;
+        auto leaf = [&](uint32_t q) -> uint64_t {
+            const uint64_t u = cpx_quot40(xp, xpd, q), pu = cpx_pi_ge2(T, u);
+            return u < y ? 2 * pu : pu;
+        };
         uint64_t ps = 0;
-        uint32_t nbuf = 0;
-        auto answer = [&](uint64_t q) {
-            const uint64_t u = cpx_udiv_leaf(xp, q);
-            const uint64_t pu = cpx_pi_dev(T, u);
-            ps += u < y ? 2 * pu : pu;
-        };
-        auto flush = [&] {
-            __syncwarp();
-            for (uint32_t j = lane; j < nbuf; j += 32) answer(qbuf[j]);
-            __syncwarp();
-            nbuf = 0;
-        };
-        for (uint64_t wb = w_beg; wb < w_end; wb += 32) {  // uniform over the warp
-            const uint64_t wq = wb + lane;
-            uint64_t qb = 0;
-            if (wq < w_end) qb = __ldg(reinterpret_cast<const ulonglong2 *>(T) + wq).x & range_mask(wq, p, qhi);
-            const uint32_t nq = (uint32_t)__popcll(qb);
-            uint32_t off;
-            const uint32_t tot = warp_place(nq, lane, off);
-            if (tot > kGABuf) {  // dense: each lane answers its own entry
-                while (qb) {
-                    const int j = __ffsll((long long)qb) - 1;
-                    qb &= qb - 1;
-                    answer(128 * wq + 2 * j + 1);
-                }
-                continue;
-            }
-            if (nbuf + tot > kGABuf) flush();
-            uint32_t kk = nbuf + off;
-            while (qb) {
-                const int j = __ffsll((long long)qb) - 1;
-                qb &= qb - 1;
-                qbuf[kk++] = (uint32_t)(128 * wq + 2 * j + 1);
-            }
-            nbuf += tot;
-        }
-        flush();
+        uint32_t t = tid;
+        for (; t + 768 < nq; t += 1024)
+            ps += (leaf(__ldg(Pq + t)) + leaf(__ldg(Pq + t + 256))) + (leaf(__ldg(Pq + t + 512)) + leaf(__ldg(Pq + t + 768)));
+        for (; t < nq; t += 256) ps += leaf(__ldg(Pq + t));
         sum += ps;
     }
     // warp total into the device sum
     const i128 t = cpx_warp_sum_i128((i128)sum);
-    if (lane == 0 && t) cpx_atomic_add_i128(acc + 2 * G_A, t);
+    if ((tid & 31) == 0 && t) cpx_atomic_add_i128(acc + 2 * G_A, t);
 }
 
 // One thread per p = P[i], i in [ir4, b3): for i < d the trivial leaves of C
@@ -170,7 +147,7 @@ void gourdon_terms(cpx_ctx *ctx, uint64_t x, uint64_t y, uint32_t c, i128 out[7]
     // A and the Sigma sums read pi(v) for v <= sqrt x and the primes to cbrt x
     TableNeed need;
     need.N = sx + 2;
-    need.P = cx + 1;
+    need.P = std::max(cx, cpx_isqrt((u128)(x / std::max<uint64_t>(xs, 2)))) + 2;  // the q of A
     grow_tables(ctx, need);
     const std::vector<uint32_t> &hP = host_primes(ctx);
     const uint32_t ir4 = (uint32_t)host_pi(hP, r4), d = (uint32_t)host_pi(hP, xs), b3 = (uint32_t)host_pi(hP, cx);
