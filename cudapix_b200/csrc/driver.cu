@@ -739,15 +739,18 @@ replan:  // again without the batch alpha when its shared sieve would not fit (b
         if (btune->offload) offload0 = btune->offload;
         if (!lbits_cap) lbits_cap = btune->lbits;
     }
-    // untuned very large queries (z >= 2^40, about x >= 1e19): 128 threads a
-    // segment (four warps over 2^18 odd numbers) visit fewer (warp, level)
-    // pairs; on a B200 the hard leaves of pi(1e20) took 6.1 s against 7.9 s
-    // with 256
-    if (!rq.threads && !ctx->hard_params_set && !btune && !(tune && tune[decade_of(xmax_all(qd))].threads)) {
+    // untuned lone queries with z >= 2^29 (about x >= 1e15): 512 threads over
+    // segments of 2^19 odd numbers (on a B200, ms of the sieve of pi(1e15),
+    // pi(1e17), pi(1.9e19): 1.6, 16.0, 540, against 1.6, 19.3, 628 with 256 over
+    // 2^18 and 1.8, 21.3, 664 with 128 over 2^18)
+    if (small && !rq.threads && !ctx->hard_params_set && !(tune && tune[decade_of(xmax_all(qd))].threads)) {
         uint64_t zmax = 0;
         for (const QD &d : qd)
             if (!d.direct) zmax = std::max(zmax, d.z);
-        if (zmax >> 40) threads = 128;
+        if (zmax >> 29) {
+            threads = 512;
+            if (!lbits_cap) lbits_cap = 19;
+        }
     }
     if (threads != 128 && threads != 256 && threads != 512 && threads != 1024)
         fail(CPX_EINVAL, "hard threads must be 128/256/512/1024");

@@ -30,12 +30,15 @@
 // sub-segments enter the hard sum and the per-unit (count, Sum(-mu)) pairs go
 // to k_hard_combine, which adds the carries between segments.
 //
-// Integer issue and the latency of a warp's chain of levels bound the kernel,
-// not memory.  Hard leaves on a B200, one level at a time with the heavy leaf
-// sets in a kernel of their own, then blocks at once, then units split by
-// their leaves and leaves found for a run of levels before they are needed:
-// pi(1e12) 0.300, 0.202, 0.205 ms; pi(1e15) 3.05, 2.43, 1.93; pi(1e17) 36.3,
-// 30.2, 22.3; pi(1.9e19) 1370, 950, 628.
+// Integer issue and the latency of a warp's chain of levels bound the kernel
+// (73% of the issue slots at pi(1e15)), not memory.  Hard leaves on a B200, ms:
+// one level at a time with the heavy leaf sets in a kernel of their own; blocks
+// at once; units split by their leaves, and leaves found for a run of levels
+// before they are needed; octets, and the segment sizes of the tuning table:
+//   pi(1e12)    0.300   0.202   0.205   0.123
+//   pi(1e15)    3.05    2.43    1.93    1.58
+//   pi(1e17)    36.3    30.2    22.3    16.0
+//   pi(1.9e19)  1370    950     628     540
 //
 // This is the sieve of lone queries and small batches.  Larger batches share
 // the sieve between queries (hard_shared.cu).
@@ -187,28 +190,28 @@ __global__ void __launch_bounds__(512, 2) k_hard(const QD *__restrict__ qd, uint
             cross_params(lp, lo_w, hi_w, lr0, li0);
         }
         // Items of each level's candidates: the primes P[k] of a prime-only level
-        // (m = q > max(mlo, p)), each a leaf, or the 4-m groups of packed mu*lpf.
-        // p^2 > y from some level on, so the group levels of a block come first.
+        // (m = q > max(mlo, p)), each a leaf, or the octets of packed mu*lpf.
+        // p^2 > y from some level on, so the octet levels of a block come first.
         const bool prime_j = (uint64_t)lp * lp > y;
         const uint32_t qa_j = lmlo > lp ? lmlo : lp;
-        uint32_t nw_j = 0, ng_j = 0, k0_j = 0;
+        uint32_t nw_j = 0, ng_j = 0, k0_j = 0, lf_j = 0;  // lf_j: its leaves at most
         if (lmhi > lmlo) {
             if (!prime_j) {
-                ng_j = ((lmhi - 1) >> 3) - ((lmlo + 1) >> 3) + 1;
+                ng_j = ((lmhi - 1) >> 4) - ((lmlo + 1) >> 4) + 1;
+                lf_j = ((lmhi - 1) >> 1) - ((lmlo + 1) >> 1) + 1;
             } else if (lmhi > qa_j) {
                 k0_j = (uint32_t)cpx_pi_ge2(Tpi, qa_j);
-                nw_j = (uint32_t)cpx_pi_ge2(Tpi, lmhi) - k0_j;
+                nw_j = lf_j = (uint32_t)cpx_pi_ge2(Tpi, lmhi) - k0_j;
             }
         }
         LvlSum *ar = area + (grp & 1) * NW * 32;
         ar[warp * 32 + lane].ms = 0;
-        // the levels' leaves at most, and about one bit in seven of a level's
-        // multiples is still set
-        const uint32_t lf_j = min(nw_j, 1u << 20) + 4 * min(ng_j, 1u << 20);
+        lf_j = min(lf_j, 1u << 20);
+        // about one bit in seven of a level's multiples is still set
         const uint32_t pmin = __shfl_sync(FULL, lp, 0);
         bool at_once = (uint64_t)pmin * kLevelWindows >= Lw;
         if (at_once) {
-            const uint32_t est = __reduce_add_sync(FULL, min(nw_j + ng_j, 1u << 26)) / us.nparts;
+            const uint32_t est = __reduce_add_sync(FULL, min(nw_j + 2 * ng_j, 1u << 26)) / us.nparts;
             at_once = (uint64_t)est * (nl * (Lw / pmin + 1) / 7 + 4) <= (uint64_t)nl * kLevelLeafEvents;
         }
         uint32_t mine_cnt = 0;
@@ -223,15 +226,42 @@ __global__ void __launch_bounds__(512, 2) k_hard(const QD *__restrict__ qd, uint
             const uint32_t k = __shfl_sync(FULL, k0_j - ex_w, jq) + f;
             return f < end ? __ldg(P + k) : 1u;
         };
-        // item f of the block's groups: its level, first m index / 4, valid m's and their signs
-        auto group_item = [&](uint32_t f, uint32_t end, uint32_t &jq, uint64_t &g4, uint32_t &neg) -> uint32_t {
+        // item f of the block's octets: its level and which octet
+        auto octet_item = [&](uint32_t f, uint32_t end, uint32_t &jq, uint32_t &o) -> Octet {
             jq = item_owner(ex_g, f);
             const uint32_t exq = __shfl_sync(FULL, ex_g, jq), pq = __shfl_sync(FULL, lp, jq);
-            const uint64_t mlq = __shfl_sync(FULL, lmlo, jq), mhq = __shfl_sync(FULL, lmhi, jq);
-            const uint64_t i_lo = (mlq + 1) >> 1, i_hi = (mhq - 1) >> 1;
-            neg = 0;
-            g4 = (i_lo >> 2) + (f - exq);
-            return f < end ? valid_group(__ldg(reinterpret_cast<const int4 *>(MU) + g4), g4, i_lo, i_hi, pq, &neg) : 0u;
+            const uint32_t i_lo = (__shfl_sync(FULL, lmlo, jq) + 1) >> 1, i_hi = (__shfl_sync(FULL, lmhi, jq) - 1) >> 1;
+            o = (i_lo >> 3) + (f - exq);
+            return load_octet(MU, o, i_lo, i_hi, pq, f < end);
+        };
+        // Gathers the leaves of the octets item(from + lane), item(from + st + lane), ..
+        // below end into the warp's buffer, which flush empties when it cannot hold
+        // a round's more, and once at the end.
+        uint32_t nbuf = 0;
+        auto gather = [&](uint32_t from, uint32_t end, uint32_t st, auto &&item, auto &&flush) {
+            for (uint32_t base = from;; base += st) {
+                const bool last = base >= end;
+                uint32_t jq = 0, o = 0;
+                const Octet t = item(last ? end : base + lane, jq, o);
+                uint32_t now = t.valid, rest = 0, tot_r = __reduce_add_sync(FULL, (uint32_t)__popc(now));
+                if (tot_r > kLeafCap) {  // a dense round goes in two halves of the octets
+                    rest = now & 0xF0u;
+                    now &= 0xFu;
+                    tot_r = __reduce_add_sync(FULL, (uint32_t)__popc(now));
+                }
+                for (;;) {
+                    if (last || nbuf + tot_r > kLeafCap) flush();
+                    if (last) return;
+                    uint32_t off_l;
+                    warp_place((uint32_t)__popc(now), lane, off_l);
+                    put_octet(t, o, now, jq, lbuf, nbuf + off_l);
+                    nbuf += tot_r;
+                    if (!__any_sync(FULL, rest != 0)) break;
+                    now = rest;
+                    rest = 0;
+                    tot_r = __reduce_add_sync(FULL, (uint32_t)__popc(now));
+                }
+            }
         };
         // bits [0, kk) of the sub-segment are the numbers up to u = xp / m
         auto leaf_bits = [&](XT xp, double xpd, uint32_t m) -> uint32_t {
@@ -241,7 +271,7 @@ __global__ void __launch_bounds__(512, 2) k_hard(const QD *__restrict__ qd, uint
         if (at_once) {
             uint32_t i = li0, w_end = pmin, cleared = 0;
             if (!(tot_w | tot_g)) {
-                cross_levels<false>(bm, cnt8, lp, i, pmin, w_end, cleared, s, CPT * 32 * warp, lane, Lw, ev, 0);
+                cross_levels(bm, cnt8, lp, i, pmin, w_end, cleared, s, CPT * 32 * warp, lane, Lw, ev, 0);
             } else {
                 // Slices of the sub-segment, as many as the bits cleared in it fill
                 // the event buffer (nearly always one): a slice's leaves have k_lo <
@@ -255,8 +285,8 @@ __global__ void __launch_bounds__(512, 2) k_hard(const QD *__restrict__ qd, uint
                         const uint32_t t = __shfl_down_sync(FULL, suf, oo);
                         if (lane + oo < 32) suf += t;
                     }
-                    const uint32_t nev = cross_levels<true>(bm, cnt8, lp, i, pmin, w_end, cleared, s, CPT * 32 * warp,
-                                                            lane, Lw, ev, kEvCap);
+                    const uint32_t nev = cross_levels(bm, cnt8, lp, i, pmin, w_end, cleared, s, CPT * 32 * warp, lane, Lw,
+                                                      ev, kEvCap);
                     const uint32_t k_hi = min(w_end - pmin, Lw);
                     if (lane < 4 && nev + lane < kEvCap) ev[nev + lane] = kEvMask;  // fills the last four
                     uint32_t off0;
@@ -289,31 +319,18 @@ __global__ void __launch_bounds__(512, 2) k_hard(const QD *__restrict__ qd, uint
                         answer(base + lane < tot_w, m, jq, true);  // mu(q) = -1
                     }
                     if (tot_g) {
-                        uint32_t nbuf = 0;
                         auto flush = [&] {
                             __syncwarp();
                             for (uint32_t j0 = 0; j0 < nbuf; j0 += 32) {
                                 const bool on = j0 + lane < nbuf;
                                 const uint2 e = on ? lbuf[j0 + lane] : make_uint2(1, 0);
-                                answer(on, e.x, e.y & 31u, (e.y >> 31) != 0);
+                                answer(on, e.x & 0x7FFFFFFFu, e.y, (e.x >> 31) != 0);
                             }
                             __syncwarp();
                             nbuf = 0;
                         };
-                        for (uint32_t base = first; base < tot_g; base += step) {
-                            uint32_t jq, neg, off_l;
-                            uint64_t g4;
-                            uint32_t vm = group_item(base + lane, tot_g, jq, g4, neg);
-                            const uint32_t tot_r = warp_place((uint32_t)__popc(vm), lane, off_l);
-                            if (nbuf + tot_r > kLeafCap) flush();
-                            for (uint32_t kk = nbuf + off_l; vm; kk++) {
-                                const int kq = __ffs(vm) - 1;
-                                vm &= vm - 1;
-                                lbuf[kk] = make_uint2((uint32_t)(2 * (4 * g4 + kq) + 1), jq | (((neg >> kq) & 1u) << 31));
-                            }
-                            nbuf += tot_r;
-                        }
-                        flush();
+                        gather(first, tot_g, step, [&](uint32_t f, uint32_t &jq, uint32_t &o) { return octet_item(f, tot_g, jq, o); },
+                               flush);
                     }
                     if (k_hi == Lw) break;
                     k_lo = k_hi;
@@ -343,25 +360,20 @@ __global__ void __launch_bounds__(512, 2) k_hard(const QD *__restrict__ qd, uint
                     if (dense) {
                         kb = k + 1;
                     } else {
-                        uint32_t nbuf = 0;
                         const uint32_t gs = __shfl_sync(FULL, ex_g, k), ws = __shfl_sync(FULL, ex_w, k);
                         const uint32_t ge = __shfl_sync(FULL, ex_g + ng_j, kb - 1),
                                        we = __shfl_sync(FULL, ex_w + nw_j, kb - 1);
-                        for (uint32_t base = gs; base < ge; base += 32) {
-                            uint32_t jq, neg, off_l;
-                            uint64_t g4;
-                            uint32_t vm = group_item(base + lane, ge, jq, g4, neg);
-                            const XT xk = shfl_xt(lxp, jq);
-                            const double xkd = (double)(uint64_t)xk;
-                            const uint32_t tot_r = warp_place((uint32_t)__popc(vm), lane, off_l);
-                            for (uint32_t t = nbuf + off_l; vm; t++) {
-                                const int kq = __ffs(vm) - 1;
-                                vm &= vm - 1;
-                                lbuf[t] = make_uint2(leaf_bits(xk, xkd, (uint32_t)(2 * (4 * g4 + kq) + 1)) |
-                                                         (((neg >> kq) & 1u) << 31),
-                                                     jq);
-                            }
-                            nbuf += tot_r;
+                        nbuf = 0;
+                        // (a run's leaves fit the buffer)
+                        gather(gs, ge, 32, [&](uint32_t f, uint32_t &jq, uint32_t &o) { return octet_item(f, ge, jq, o); },
+                               [] {});
+                        __syncwarp();
+                        for (uint32_t t0 = 0; t0 < nbuf; t0 += 32) {
+                            const bool on = t0 + lane < nbuf;
+                            const uint2 e = on ? lbuf[t0 + lane] : make_uint2(1, 0);
+                            const XT xk = shfl_xt(lxp, e.y);
+                            if (on)
+                                lbuf[t0 + lane].x = leaf_bits(xk, (double)(uint64_t)xk, e.x & 0x7FFFFFFFu) | (e.x & 0x80000000u);
                         }
                         for (uint32_t base = ws; base < we; base += 32) {
                             uint32_t jq;
@@ -417,41 +429,27 @@ __global__ void __launch_bounds__(512, 2) k_hard(const QD *__restrict__ qd, uint
                             S += (int64_t)count(leaf_bits(xp, xpd, __ldg(Pk + f)));
                             msl += 1;
                         }
-                        // groups (the next round's are loaded before this round's are answered)
-                        const uint32_t mlo = __shfl_sync(FULL, lmlo, k), mhi = __shfl_sync(FULL, lmhi, k);
-                        const uint64_t i_lo = ((uint64_t)mlo + 1) >> 1, i_hi = ((uint64_t)mhi - 1) >> 1;
-                        uint32_t nbuf = 0;
-                        auto flush = [&] {
-                            __syncwarp();
-                            for (uint32_t t = lane; t < nbuf; t += 32) {
-                                const uint2 e = lbuf[t];
-                                const uint32_t cv = count(leaf_bits(xp, xpd, e.x));
-                                S += e.y ? (int64_t)cv : -(int64_t)cv;
-                                msl += e.y ? 1 : -1;
-                            }
-                            __syncwarp();
+                        if (ng > first) {
+                            const uint32_t i_lo = (__shfl_sync(FULL, lmlo, k) + 1) >> 1,
+                                           i_hi = (__shfl_sync(FULL, lmhi, k) - 1) >> 1;
                             nbuf = 0;
-                        };
-                        auto four = [&](uint32_t g) -> int4 {
-                            return g < ng ? __ldg(reinterpret_cast<const int4 *>(MU) + (i_lo >> 2) + g)
-                                          : make_int4(0, 0, 0, 0);
-                        };
-                        int4 next = four(first + lane);
-                        for (uint32_t base = first; base < ng; base += step) {
-                            const uint64_t g4 = (i_lo >> 2) + base + lane;
-                            uint32_t neg = 0, off_l;
-                            uint32_t vm = valid_group(next, g4, i_lo, i_hi, p, &neg);
-                            next = four(base + step + lane);
-                            const uint32_t tot_r = warp_place((uint32_t)__popc(vm), lane, off_l);
-                            if (nbuf + tot_r > kLeafCap) flush();
-                            for (uint32_t t = nbuf + off_l; vm; t++) {
-                                const int kq = __ffs(vm) - 1;
-                                vm &= vm - 1;
-                                lbuf[t] = make_uint2((uint32_t)(2 * (4 * g4 + kq) + 1), (neg >> kq) & 1u);
-                            }
-                            nbuf += tot_r;
+                            auto flush = [&] {
+                                __syncwarp();
+                                for (uint32_t t = lane; t < nbuf; t += 32) {
+                                    const uint32_t e = lbuf[t].x, cv = count(leaf_bits(xp, xpd, e & 0x7FFFFFFFu));
+                                    S += e >> 31 ? (int64_t)cv : -(int64_t)cv;
+                                    msl += e >> 31 ? 1 : -1;
+                                }
+                                __syncwarp();
+                                nbuf = 0;
+                            };
+                            gather(first, ng, step,
+                                   [&](uint32_t f, uint32_t &, uint32_t &o) {
+                                       o = (i_lo >> 3) + f;
+                                       return load_octet(MU, o, i_lo, i_hi, p, f < ng);
+                                   },
+                                   flush);
                         }
-                        flush();
                     }
                     const int32_t ms = __reduce_add_sync(FULL, msl);
                     if (lane == k) ar[warp * 32 + k].ms = ms;

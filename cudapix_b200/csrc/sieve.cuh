@@ -133,18 +133,17 @@ static __device__ __noinline__ void snapshot_chunks(uint4 *sb, uint32_t *spre, c
 }
 
 // The valid m of one 16-byte group of packed mu*lpf (4 odd m, indices 4g..4g+3
-// within [i_lo, i_hi]): squarefree with lpf > p.  Bit k of *neg: mu(m) = -1.
-__device__ __forceinline__ uint32_t valid_group(int4 v4, uint64_t g, uint64_t i_lo, uint64_t i_hi, uint32_t p,
+// within [i_lo, i_hi], below 2^30): squarefree with lpf > p.  Bit k of *neg: mu(m) = -1.
+__device__ __forceinline__ uint32_t valid_group(int4 v4, uint32_t g, uint32_t i_lo, uint32_t i_hi, uint32_t p,
                                                 uint32_t *neg)
 {
     const int32_t vals[4] = {v4.x, v4.y, v4.z, v4.w};
     uint32_t vm = 0, ng = 0;
 #pragma unroll
     for (int k = 0; k < 4; k++) {
-        const uint64_t i = 4 * g + k;
+        const uint32_t i = 4 * g + k;
         const int32_t v = vals[k];
-        const uint32_t av = (uint32_t)(v > 0 ? v : -v);
-        if (i >= i_lo && i <= i_hi && v != 0 && av > p) {
+        if (i >= i_lo && i <= i_hi && (uint32_t)abs(v) > p) {  // (v = 0: mu(m) = 0)
             vm |= 1u << k;
             if (v < 0) ng |= 1u << k;
         }
@@ -296,11 +295,12 @@ __device__ __forceinline__ uint32_t cross_off(uint32_t *bm, uint8_t *cnt8, uint3
 
 // A leaf quotient x/(p m) = xp / m of a leaf in a sub-segment that ends at
 // or below 2^41 (q41, so the quotient is below 2^41): cpx_quot40 when xp <
-// 2^53 (xpd = xp as a double, exact), else cpx_qdiv.
+// 2^63 (xpd = xp as a double), else cpx_qdiv, out of line (rare, and long).
+template <class XT> static __device__ __noinline__ uint64_t leaf_quot_wide(XT xp, uint64_t m) { return (uint64_t)cpx_qdiv(xp, m); }
 template <class XT> __device__ __forceinline__ uint64_t leaf_quot(XT xp, double xpd, uint64_t m, bool q41)
 {
-    if (q41 && ((u128)xp >> 53) == 0) return cpx_quot40((uint64_t)xp, xpd, (uint32_t)m);
-    return (uint64_t)cpx_qdiv(xp, m);
+    if (q41 && ((u128)xp >> 63) == 0) return cpx_quot40((uint64_t)xp, xpd, (uint32_t)m);
+    return leaf_quot_wide<XT>(xp, m);
 }
 
 // Survivors among bits 0..jb of one 16-byte bitmap chunk, without a branch.

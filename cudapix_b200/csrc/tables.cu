@@ -652,7 +652,7 @@ void ensure_mulpf(cpx_ctx *ctx, uint64_t ymax)
         tb.MU = nullptr;
         tb.mu_n = 0;
     }
-    CPX_CUDA(cudaMalloc(&tb.MU, len * 4));
+    CPX_CUDA(cudaMalloc(&tb.MU, (len + 16) * 4));  // the last octet may be read whole
     mulpf_sieve(ctx, 0, 2 * len, nullptr, nullptr, nullptr, tb.MU);
     tb.mu_n = 2 * len - 1;
     tb.version++;
