@@ -38,9 +38,15 @@ __host__ __device__ __forceinline__ size_t counts_smem(uint32_t lbits)
     return L / 8 + (((L / 128) + 15) & ~size_t(15));
 }
 
-// gathered leaves per warp: 256, or 128 for 32 warps (2^20 bits, 1024
-// threads, fit 227 KB of shared memory)
-__host__ __device__ __forceinline__ uint32_t leaf_cap(uint32_t threads) { return threads >= 1024 ? 128u : kLeafBuf; }
+// leaves a warp gathers before answering them 32 at a time
+constexpr uint32_t kGatherCap = 128;
+
+// bytes of the unit's hard sums: per (group, slot) one 64-bit word a warp, or
+// one 128-bit value (at most eight warps keep words of their own)
+__host__ __device__ __forceinline__ size_t sum_bytes(uint32_t threads)
+{
+    return (size_t)kBlockMax * kGroupMax * (threads <= 256 ? (threads / 32 < 2 ? 2 : threads / 32) * 8 : 16);
+}
 
 // shared memory of k_hard_shared
 __host__ __device__ __forceinline__ size_t shared_smem(uint32_t lbits, uint32_t threads)
@@ -48,11 +54,11 @@ __host__ __device__ __forceinline__ size_t shared_smem(uint32_t lbits, uint32_t 
     size_t o = counts_smem(lbits);
     o += ((size_t(1) << lbits) / 128) * 2;         // chunk prefixes within their lane
     o += threads * 4;                              // lane prefixes
-    o += (threads / 32) * leaf_cap(threads) * 8;   // gathered leaves: m, query | (mu(m) = -1) << 31
+    o += (threads / 32) * kGatherCap * 8;          // gathered leaves: m, query | (mu(m) = -1) << 31
     o += (threads / 32) * kGroupMax * 16;  // x/p of the group's queries, per warp
     o += (threads / 32) * kGroupMax * 12;  // per-warp, per-query level sums and Sum(-mu)
     o += kBlockMax * kGroupMax * 12;       // per (group, slot): query, y, level threshold
-    o += kBlockMax * kGroupMax * 16;       // per (group, slot): the hard sum over the unit
+    o += sum_bytes(threads);               // per (group, slot): the hard sum over the unit
     return o;
 }
 
@@ -258,6 +264,13 @@ constexpr uint32_t kLaneEntries = 128;
 // Sum(-mu) for the query of its last leaf and adds them into the warp's
 // per-query slots when the query changes; at the end of the level lane j
 // adds slot j into its query's unit sum as sum + carry * Sum(-mu).
+// A lane that answers its own query reads prime m from the prime list by rank
+// (two table lookups a level) and adds into its warp's own word of the unit's
+// sums: the 4096-query batch 20.3 -> 17.1 ms of this kernel, 1024 queries in
+// [1e10, 1e15] 29.8 -> 24.6, against prime m found bit by bit in pi-table words
+// and 128-bit sums by shared-memory atomics.  With four warps a scheduler (the
+// bitmaps fill the shared memory) it is bound by the latency of a warp's chain:
+// 58% of the issue slots.
 // The launch bounds (at most TMAX threads, at least MINB blocks per SM) set
 // the register budget: 65536 / (TMAX MINB) a thread, 64 when 32 warps share
 // an SM and 128 (no spills) when 16 do.  The launch takes the variant whose
@@ -269,10 +282,10 @@ constexpr uint32_t kLaneEntries = 128;
         uint32_t nlv, const uint64_t *__restrict__ carry, unsigned long long *__restrict__ acc,                   \
         HardJob *__restrict__ jobs, unsigned int *__restrict__ njobs, uint64_t *__restrict__ job_units,          \
         unsigned char *__restrict__ snap, unsigned int *__restrict__ nsnap, uint32_t max_jobs, uint32_t lbits_sub, \
-        uint32_t offload_min, const XT *__restrict__ gxp, const uint2 *__restrict__ gae
+        uint32_t offload_min, const XT *__restrict__ gxp, const uint2 *__restrict__ gae, uint32_t narrow
 #define CPX_HS_ARGS                                                                                             \
     qd, grp, units, total, lbits, c, P, np, MU, Tpi, lvl_off, nlv, carry, acc, jobs, njobs, job_units, snap, \
-        nsnap, max_jobs, lbits_sub, offload_min, gxp, gae
+        nsnap, max_jobs, lbits_sub, offload_min, gxp, gae, narrow
 
 // one unit of the shared sieve, by one CTA: a segment and up to kBlockMax
 // consecutive groups (z descending), packed as seg << 32 | g0 << 4 | (n - 1).
@@ -318,7 +331,7 @@ template <class XT> __device__ __forceinline__ void hard_shared_unit(uint64_t un
     uint32_t *wl = reinterpret_cast<uint32_t *>(sp + o) + 32 * warp;  // this warp's lane prefixes
     o += T * 4;
     uint2 *lbuf0 = reinterpret_cast<uint2 *>(sp + o);
-    const uint32_t cap = leaf_cap(T);
+    constexpr uint32_t cap = kGatherCap;
     uint2 *lbuf = lbuf0 + cap * warp;
     o += NW * cap * 8;
     XT *s_xp = reinterpret_cast<XT *>(sp + o) + 32 * warp;  // x/p of each query at the current level
@@ -327,8 +340,15 @@ template <class XT> __device__ __forceinline__ void hard_shared_unit(uint64_t un
     o += NW * 32 * 8;
     int *s_ms = reinterpret_cast<int *>(sp + o) + 32 * warp;
     o += NW * 32 * 4;
-    // per (group, slot) of the block: the query, its y and its level
-    // threshold, and its hard sum over the unit (two words, added by atomics)
+    // per (group, slot) of the block: the query, its y and its level threshold,
+    // and its hard sum over the unit: with every x < 2^60 (narrow) a 64-bit word
+    // of each warp, which only the slot's lane adds to, else a 128-bit value the
+    // warps add to by atomics (64-bit atomics on shared memory are
+    // compare-and-swap loops).  A warp's word cannot overflow: at a level its
+    // leaves number at most xp / lo_w and count at most hi_w <= 2 lo_w numbers
+    // each, so they sum to at most 2 x / p_b, and 2 x times the sum of 1/p over the
+    // primes 3 <= p < 2^16 is below 4.4 x; in the sub-segment at 0, to less than
+    // y hi_w <= 2^52 at each of the at most 229 levels.
     uint32_t *s_qj = reinterpret_cast<uint32_t *>(sp + o);
     uint32_t *s_yj = s_qj + kBlockMax * 32;
     uint32_t *s_pt = s_yj + kBlockMax * 32;
@@ -355,9 +375,13 @@ template <class XT> __device__ __forceinline__ void hard_shared_unit(uint64_t un
         s_qj[t] = qv;
         s_yj[t] = yv;
         s_pt[t] = pt;
-        s_acc[2 * t] = 0;
-        s_acc[2 * t + 1] = 0;
     }
+    for (uint32_t t = tid; t < sum_bytes(T) / 8; t += T) s_acc[t] = 0;
+    unsigned long long *w_acc = s_acc + kBlockMax * 32 * warp;  // this warp's words (narrow)
+    auto add_sum = [&](uint32_t t, int64_t sum, uint64_t carry, int32_t ms) {
+        if (narrow) w_acc[t] += (unsigned long long)sum + carry * (unsigned long long)(int64_t)ms;
+        else cpx_atomic_add_i128(s_acc + 2 * t, (i128)sum + (i128)carry * (i128)ms);
+    };
     __syncthreads();
 
     const uint32_t c0 = CPT * tid, cw0 = c0 - CPT * 32 * warp;
@@ -436,21 +460,17 @@ template <class XT> __device__ __forceinline__ void hard_shared_unit(uint64_t un
                 const uint64_t C = __shfl_sync(FULL, lC, k);  // survivors below the sub-segment
                 const bool prime_j = pp > yj;  // m must be a prime q > max(mlo, p)
                 const uint32_t qa_j = mlo > p ? mlo : p;
-                uint64_t work = 0;
+                uint32_t work = 0;
                 if (act)
-                    work = prime_j ? 8 * ((((uint64_t)mhi - 1) >> 7) - (qa_j >> 7) + 1)
-                                   : ((((uint64_t)mhi - 1) >> 1) - (((uint64_t)mlo + 1) >> 1) + 1);
+                    work = prime_j ? 8 * (((mhi - 1) >> 7) - (qa_j >> 7) + 1) : ((mhi - 1) >> 1) - ((mlo + 1) >> 1) + 1;
                 // heavy sets to k_hard_leaves, one snapshot for the warp's level
                 bool off_j = act && max_jobs && offload_min && work >= offload_min;
                 if (__any_sync(FULL, off_j))
                     off_j = offload_sets<XT>(off_j, lane, qj, b, p, prime_j, qa_j, mlo, mhi, work, lo_w, C, xp, bm, cnt8,
                                              cw0, c0, CPT, s, wl[lane], jobs, njobs, job_units, snap, nsnap, max_jobs,
                                              lbits_sub);
-                const uint32_t nw_j =
-                    (act && !off_j && prime_j) ? (uint32_t)((((uint64_t)mhi - 1) >> 7) - (qa_j >> 7) + 1) : 0u;
-                uint32_t ng_j = 0;
-                if (act && !off_j && !prime_j)
-                    ng_j = (uint32_t)(((((uint64_t)mhi - 1) >> 1) >> 2) - ((((uint64_t)mlo + 1) >> 1) >> 2) + 1);
+                const uint32_t nw_j = (act && !off_j && prime_j) ? ((mhi - 1) >> 7) - (qa_j >> 7) + 1 : 0u;
+                const uint32_t ng_j = (act && !off_j && !prime_j) ? ((mhi - 1) >> 3) - ((mlo + 1) >> 3) + 1 : 0u;
                 if (!__any_sync(FULL, nw_j > kLaneEntries || ng_j > kLaneEntries)) {
                     // a sparse level (the common case: about one leaf per query;
                     // at most kLaneEntries table entries or 4-m groups each):
@@ -458,19 +478,21 @@ template <class XT> __device__ __forceinline__ void hard_shared_unit(uint64_t un
                     int64_t sv = 0;
                     int32_t sm = 0;
                     const double xpd = (double)(uint64_t)xp;
-                    for (uint32_t k2 = 0; k2 < nw_j; k2++) {
-                        const uint64_t wq = (qa_j >> 7) + k2;
-                        uint64_t qb = __ldg(reinterpret_cast<const ulonglong2 *>(Tpi) + wq).x & range_mask(wq, qa_j, mhi);
-                        while (qb) {
-                            const int jb = __ffsll((long long)qb) - 1;
-                            qb &= qb - 1;
-                            sv += sub_count(hq(xp, xpd, 128 * wq + 2 * jb + 1));  // mu(q) = -1
-                            sm += 1;
+                    if (nw_j) {
+                        // prime m: the primes P[k] of (qa, mhi], a leaf each
+                        const uint32_t ka = (uint32_t)cpx_pi_ge2(Tpi, qa_j), ke = (uint32_t)cpx_pi_ge2(Tpi, mhi);
+                        uint32_t k2 = ka, cs = 0;
+                        for (; k2 + 1 < ke; k2 += 2) {
+                            const uint32_t m0 = __ldg(P + k2), m1 = __ldg(P + k2 + 1);
+                            sv += sub_count(hq(xp, xpd, m0)) + sub_count(hq(xp, xpd, m1));  // mu(q) = -1
                         }
+                        if (k2 < ke) cs = sub_count(hq(xp, xpd, __ldg(P + k2)));
+                        sv += cs;
+                        sm = (int32_t)(ke - ka);
                     }
-                    const uint64_t i_lo = ((uint64_t)mlo + 1) >> 1, i_hi = ((uint64_t)mhi - 1) >> 1;
+                    const uint32_t i_lo = (mlo + 1) >> 1, i_hi = (mhi - 1) >> 1;
                     for (uint32_t k2 = 0; k2 < ng_j; k2++) {
-                        const uint64_t g4 = (i_lo >> 2) + k2;
+                        const uint32_t g4 = (i_lo >> 2) + k2;
                         uint32_t neg = 0;
                         uint32_t vm =
                             valid_group(__ldg(reinterpret_cast<const int4 *>(MU) + g4), g4, i_lo, i_hi, p, &neg);
@@ -487,7 +509,7 @@ template <class XT> __device__ __forceinline__ void hard_shared_unit(uint64_t un
                             }
                         }
                     }
-                    if (sv || sm) cpx_atomic_add_i128(s_acc + 2 * tq, (i128)sv + (i128)C * (i128)sm);
+                    if (sv || sm) add_sum(tq, sv, C, sm);
                     __syncwarp();
                 } else {
                 // running sums of the query of this lane's last leaf
@@ -605,8 +627,7 @@ template <class XT> __device__ __forceinline__ void hard_shared_unit(uint64_t un
                 __syncwarp();
                 // the level's sums of this lane's query: Sum(-mu)(carry + count)
                 if (lane < nq) {
-                    const i128 v = (i128)(int64_t)s_sum[lane] + (i128)C * (i128)s_ms[lane];
-                    if (v) cpx_atomic_add_i128(s_acc + 2 * tq, v);
+                    add_sum(tq, (int64_t)s_sum[lane], C, s_ms[lane]);
                     s_sum[lane] = 0;
                     s_ms[lane] = 0;
                 }
@@ -623,7 +644,12 @@ template <class XT> __device__ __forceinline__ void hard_shared_unit(uint64_t un
     __syncthreads();  // every warp is past its levels: the block's sums are complete
     for (uint32_t t = tid; t < ngr * 32; t += T) {
         if (s_qj[t] == 0xFFFFFFFFu) continue;
-        const i128 v = (i128)(((u128)s_acc[2 * t + 1] << 64) | s_acc[2 * t]);
+        i128 v = 0;
+        if (narrow) {
+            for (uint32_t k = 0; k < NW; k++) v += (i128)(int64_t)s_acc[kBlockMax * 32 * k + t];
+        } else {
+            v = (i128)(((u128)s_acc[2 * t + 1] << 64) | s_acc[2 * t]);
+        }
         if (v) acc_add(acc, s_qj[t], ACC_HARD, v);
     }
 }
@@ -703,7 +729,8 @@ template <class XT> static void shared_go(cpx_ctx *ctx, const Plan &pl)
             kern<<<grid, T, smem, ctx->stream>>>(pl.unit_next, pl.qd, pl.grp, pl.units, pl.n_gunits, pl.sh_lbits, pl.c, tb.P,
                 (uint32_t)tb.prm_n, tb.MU, tb.T, pl.lvl_off, pl.sh_nlv, pl.carry, pl.acc, pl.jobs, pl.njobs,
                 pl.job_units, pl.snap, pl.nsnap, pl.max_jobs, lbits_sub,
-                (uint32_t)std::min<uint64_t>(pl.offload_min, 0xFFFFFFFFull), gxp, pl.gae);
+                (uint32_t)std::min<uint64_t>(pl.offload_min, 0xFFFFFFFFull), gxp, pl.gae,
+                (uint32_t)(T <= 256 && (pl.sh_xmax >> 60) == 0));
         };
         const int fit = shared_blocks_per_sm(ctx, pl.sh_lbits, T);
         if (T > 512) go(k_hard_shared<XT, 1024, 1>, 1);
