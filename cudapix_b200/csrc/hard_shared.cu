@@ -242,35 +242,19 @@ static __device__ __noinline__ bool offload_sets(bool off_j, uint32_t lane, uint
     return off_j;
 }
 
-// Candidate entries (pi-table words or 4-m groups) a lane answers itself;
-// above it on any lane the warp gathers the level's leaves (on the B200 the
-// 4096-query batch took 49.0 / 46.0 / 41.4 / 40.9 ms of this kernel with 8 /
-// 16 / 32 / 64 when each unit held one group; with blocks of groups 20.9 /
-// 20.5 / 20.4 ms with 32 / 64 / 128)
-constexpr uint32_t kLaneEntries = 128;
-
 // (3) One CTA per unit: a segment and a block of up to kBlockMax groups.  Per
 // level and group, the lanes hold one query each: its x/p and candidate range
-// in the warp's sub-segment.  When no query has more than kLaneEntries
-// candidate table entries (98% of the visits of the 4096-query batch, with
-// about 1.3 entries a query), each lane answers its own query's leaves and
-// adds them into the query's slot of the unit's sums.
-// Otherwise the warp walks the candidates of all the group's queries as one
-// sequence (pi-table words of the prime-only levels, then 4-m groups of
-// packed mu*lpf of the others), 32 words at a time, each lane finding its
-// word's query by a binary search over the warp's exclusive word counts; the
-// leaves found go to the warp's buffer (m, query | (mu(m) = -1) << 31) and
-// are answered 32 at a time.  Each lane keeps a running Sum(-mu) * count and
-// Sum(-mu) for the query of its last leaf and adds them into the warp's
-// per-query slots when the query changes; at the end of the level lane j
+// in the warp's sub-segment.  When the queries have about as many items (primes
+// m or 4-m groups) each, or few, each lane answers its own query's and adds
+// them into the query's slot of the unit's sums.  Else (a group of few queries,
+// or of very different ones) the warp walks the items of all the group's
+// queries as one sequence, 32 at a time, each lane finding its item's query by a
+// binary search over the warp's exclusive item counts: a prime is answered at
+// once; the leaves of 4-m groups go to the warp's buffer (m, query | (mu(m) =
+// -1) << 31) and are answered 32 at a time.  Each lane keeps a running Sum(-mu) *
+// count and Sum(-mu) for the query of its last leaf and adds them into the
+// warp's per-query slots when the query changes; at the end of the level lane j
 // adds slot j into its query's unit sum as sum + carry * Sum(-mu).
-// A lane that answers its own query reads prime m from the prime list by rank
-// (two table lookups a level) and adds into its warp's own word of the unit's
-// sums: the 4096-query batch 20.3 -> 17.1 ms of this kernel, 1024 queries in
-// [1e10, 1e15] 29.8 -> 24.6, against prime m found bit by bit in pi-table words
-// and 128-bit sums by shared-memory atomics.  With four warps a scheduler (the
-// bitmaps fill the shared memory) it is bound by the latency of a warp's chain:
-// 58% of the issue slots.
 // The launch bounds (at most TMAX threads, at least MINB blocks per SM) set
 // the register budget: 65536 / (TMAX MINB) a thread, 64 when 32 warps share
 // an SM and 128 (no spills) when 16 do.  The launch takes the variant whose
@@ -469,27 +453,32 @@ template <class XT> __device__ __forceinline__ void hard_shared_unit(uint64_t un
                     off_j = offload_sets<XT>(off_j, lane, qj, b, p, prime_j, qa_j, mlo, mhi, work, lo_w, C, xp, bm, cnt8,
                                              cw0, c0, CPT, s, wl[lane], jobs, njobs, job_units, snap, nsnap, max_jobs,
                                              lbits_sub);
-                const uint32_t nw_j = (act && !off_j && prime_j) ? ((mhi - 1) >> 7) - (qa_j >> 7) + 1 : 0u;
+                // the primes P[ka_j] .. of (qa, mhi], a leaf each, or 4-m groups
+                uint32_t ka_j = 0, np_j = 0;
+                if (act && !off_j && prime_j) {
+                    ka_j = (uint32_t)cpx_pi_ge2(Tpi, qa_j);
+                    np_j = (uint32_t)cpx_pi_ge2(Tpi, mhi) - ka_j;
+                }
                 const uint32_t ng_j = (act && !off_j && !prime_j) ? ((mhi - 1) >> 3) - ((mlo + 1) >> 3) + 1 : 0u;
-                if (!__any_sync(FULL, nw_j > kLaneEntries || ng_j > kLaneEntries)) {
-                    // a sparse level (the common case: about one leaf per query;
-                    // at most kLaneEntries table entries or 4-m groups each):
-                    // each lane answers its own query's candidates
+                const uint32_t it_j = np_j + ng_j;
+                const uint32_t it_max = __reduce_max_sync(FULL, it_j), it_sum = __reduce_add_sync(FULL, it_j);
+                if (32ull * it_max <= 3ull * it_sum + 128) {
+                    // The queries have about as many items each, or few: each lane
+                    // answers its own query's.  (On a B200, thirty batches of 6 to
+                    // 3571 queries, their geometric mean against the word-by-word
+                    // kernel: 1.34 / 1.40 / 1.40 / 1.37 / 1.21 times as fast with 2 /
+                    // 3 / 4 / 6 / 10 here; the 4096-query batch does not mind.)
                     int64_t sv = 0;
                     int32_t sm = 0;
                     const double xpd = (double)(uint64_t)xp;
-                    if (nw_j) {
-                        // prime m: the primes P[k] of (qa, mhi], a leaf each
-                        const uint32_t ka = (uint32_t)cpx_pi_ge2(Tpi, qa_j), ke = (uint32_t)cpx_pi_ge2(Tpi, mhi);
-                        uint32_t k2 = ka, cs = 0;
-                        for (; k2 + 1 < ke; k2 += 2) {
-                            const uint32_t m0 = __ldg(P + k2), m1 = __ldg(P + k2 + 1);
-                            sv += sub_count(hq(xp, xpd, m0)) + sub_count(hq(xp, xpd, m1));  // mu(q) = -1
-                        }
-                        if (k2 < ke) cs = sub_count(hq(xp, xpd, __ldg(P + k2)));
-                        sv += cs;
-                        sm = (int32_t)(ke - ka);
+                    const uint32_t *Pk = P + ka_j;
+                    uint32_t k1 = 0;
+                    for (; k1 + 1 < np_j; k1 += 2) {
+                        const uint32_t m0 = __ldg(Pk + k1), m1 = __ldg(Pk + k1 + 1);
+                        sv += sub_count(hq(xp, xpd, m0)) + sub_count(hq(xp, xpd, m1));  // mu(q) = -1
                     }
+                    if (k1 < np_j) sv += sub_count(hq(xp, xpd, __ldg(Pk + k1)));
+                    sm = (int32_t)np_j;
                     const uint32_t i_lo = (mlo + 1) >> 1, i_hi = (mhi - 1) >> 1;
                     for (uint32_t k2 = 0; k2 < ng_j; k2++) {
                         const uint32_t g4 = (i_lo >> 2) + k2;
@@ -557,38 +546,17 @@ template <class XT> __device__ __forceinline__ void hard_shared_unit(uint64_t un
                     return jq;
                 };
                 {
-                    // prime-only levels: pi-table words of (max(mlo, p), mhi]
+                    // prime-only levels: the primes of all queries, one a lane
                     uint32_t ex_j;
-                    const uint32_t tot_w = warp_place(nw_j, lane, ex_j);
+                    const uint32_t tot_w = warp_place(np_j, lane, ex_j);
                     for (uint32_t base = 0; base < tot_w; base += 32) {
                         const uint32_t f = base + lane;
                         const uint32_t jq = owner(ex_j, f);
-                        const uint32_t exq = __shfl_sync(FULL, ex_j, jq);
-                        const uint64_t qaq = __shfl_sync(FULL, qa_j, jq), mhq = __shfl_sync(FULL, mhi, jq);
-                        uint64_t qb = 0, wq = 0;
+                        const uint32_t k = __shfl_sync(FULL, ka_j - ex_j, jq) + f;
                         if (f < tot_w) {
-                            wq = (qaq >> 7) + (f - exq);
-                            qb = __ldg(reinterpret_cast<const ulonglong2 *>(Tpi) + wq).x & range_mask(wq, qaq, mhq);
-                        }
-                        uint32_t off;
-                        const uint32_t tot_r = warp_place((uint32_t)__popcll(qb), lane, off);
-                        if (tot_r > cap) {  // a dense round: each lane answers its own word
                             const XT xq = s_xp[jq];
-                            while (qb) {
-                                const int jb = __ffsll((long long)qb) - 1;
-                                qb &= qb - 1;
-                                put(jq, sub_count(hq(xq, (double)(uint64_t)xq, 128 * wq + 2 * jb + 1)), true);  // mu(q) = -1
-                            }
-                            continue;
+                            put(jq, sub_count(hq(xq, (double)(uint64_t)xq, __ldg(P + k))), true);  // mu(q) = -1
                         }
-                        if (nbuf + tot_r > cap) flush();
-                        uint32_t kk = nbuf + off;
-                        while (qb) {
-                            const int jb = __ffsll((long long)qb) - 1;
-                            qb &= qb - 1;
-                            lbuf[kk++] = make_uint2((uint32_t)(128 * wq + 2 * jb + 1), jq | 0x80000000u);
-                        }
-                        nbuf += tot_r;
                     }
                 }
                 {
