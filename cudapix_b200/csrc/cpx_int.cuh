@@ -269,17 +269,27 @@ __device__ __forceinline__ uint64_t cpx_quot40(uint64_t n, double nd, uint32_t d
     return cpx_quot40_core<uint64_t>(n, nd, d, cpx_rcp_approx(d));
 }
 
-// pi(floor(n / d)) of an easy leaf whose dividend n = x/p is below 2^40, with
-// d = q < 2^31 and a quotient u below 2^30 (u < sqrt(x), x < 2^60 when x/p <
-// 2^40), by cpx_quot40_small.
-// u >= 2; pi(u) = 1 + entry prefix + bits 0..j of the entry's bitmap,
-// j = ((u - 1) mod 128) / 2.
-__device__ __forceinline__ uint64_t cpx_pi_quot40(const cpx_pient *__restrict__ T, uint64_t n, double nd, uint32_t d)
+// the same with a quotient below 2^32 - 1
+__device__ __forceinline__ uint32_t cpx_quot40_u32(uint64_t n, double nd, uint32_t d)
 {
-    const uint32_t m = cpx_quot40_small(n, nd, d, cpx_rcp_approx(d)) - 1;
+    return cpx_quot40_core<uint32_t>(n, nd, d, cpx_rcp_approx(d));
+}
+
+// pi(u) for 2 <= u from the compressed table: 1 + entry prefix + bits 0..j of
+// the entry's bitmap, j = ((u - 1) mod 128) / 2
+__device__ __forceinline__ uint64_t cpx_pi_ge2_u32(const cpx_pient *__restrict__ T, uint32_t u)
+{
+    const uint32_t m = u - 1;
     const ulonglong2 e = __ldg(reinterpret_cast<const ulonglong2 *>(T) + (m >> 7));
     const uint32_t j = (m & 127u) >> 1;
     return 1 + e.y + (uint64_t)__popcll(e.x << (63 - j));
+}
+
+// pi(floor(n / d)) of an easy leaf, n = x/p < 2^63, with d = q < 2^31 and a
+// quotient 2 <= u < 2^31 - 1, by cpx_quot40_small.
+__device__ __forceinline__ uint64_t cpx_pi_quot40(const cpx_pient *__restrict__ T, uint64_t n, double nd, uint32_t d)
+{
+    return cpx_pi_ge2_u32(T, cpx_quot40_small(n, nd, d, cpx_rcp_approx(d)));
 }
 
 // floor(n / d) for n < 2^53 and a quotient below 2^44, d < 2^32, nd = n as a
