@@ -433,7 +433,7 @@ __global__ void k_easy_count(const QD *__restrict__ qd, uint32_t Q, const uint64
 // kEasySparse consecutive primes q of one p (lane l takes k = k0 + l, k0 + l +
 // 32, ...); a clustered chunk is kEasyClu consecutive u primes of one p.
 template <class XT>
-__global__ void __launch_bounds__(kThreads) k_easy(const QD *__restrict__ qd, uint32_t Q,
+__global__ void __launch_bounds__(kThreads, 4) k_easy(const QD *__restrict__ qd, uint32_t Q,
                                                    const uint64_t *__restrict__ pre, uint64_t total_units,
                                                    const uint64_t *__restrict__ off,
                                                    const uint32_t *__restrict__ P, uint64_t prm_max,
@@ -444,11 +444,16 @@ __global__ void __launch_bounds__(kThreads) k_easy(const QD *__restrict__ qd, ui
     const int lane = threadIdx.x & 31;
     const WarpSlice sl = warp_slice(off[total_units]);
     LaneAcc a;
-    // decoded state of the current p, kept across its consecutive chunks
+    // decoded state of the current p, kept across its consecutive chunks; the
+    // plan in shared memory, so that its eighteen registers hold leaves instead
+    // (spilled before: k_easy of pi(1.9e19) 259 -> 211 ms, pi(1e17) 7.0 -> 6.7; 48
+    // or 40 registers a thread and more warps: 219 and 218, 6.6 and 6.45, and 12.1
+    // and 12.2 ms on the batch of 4096 where 64 registers take 11.7)
+    __shared__ EasyP s_e[kThreads / 32];
+    EasyP &e = s_e[threadIdx.x >> 5];
     uint64_t c_unit = ~0ull, c_first = 0, c_last = 0, b = 0;
     uint32_t q = 0;
     XT xp = 0;
-    EasyP e = {};
     for (uint64_t ch = sl.u0; ch < sl.u1; ch++) {
         if (ch > c_last || c_unit == ~0ull) {
             // the unit of chunk ch: a binary search for the slice's first
@@ -465,10 +470,11 @@ __global__ void __launch_bounds__(kThreads) k_easy(const QD *__restrict__ qd, ui
                 do c_unit++;
                 while (__ldg(off + c_unit + 1) <= ch);
             }
+            EasyP pl = {};
             if (rec) {
                 const EasyRec r = rec[c_unit];
                 xp = (XT)r.xp;
-                easy_unpack(r, e);
+                easy_unpack(r, pl);
                 b = r.b;
                 q = r.q;
             } else {
@@ -476,10 +482,13 @@ __global__ void __launch_bounds__(kThreads) k_easy(const QD *__restrict__ qd, ui
                 const QD &d = qd[q];
                 const uint64_t i = c_unit - __ldg(pre + q);
                 b = d.c + 1 + i;  // p = p_b
-                easy_plan<XT>(xload<XT>(d), d.y, __ldg(P + d.c + i), prm_max, T, xp, e);
+                easy_plan<XT>(xload<XT>(d), d.y, __ldg(P + d.c + i), prm_max, T, xp, pl);
             }
             c_first = __ldg(off + c_unit);
-            c_last = c_first + e.nsp + e.ncl - 1;
+            c_last = c_first + pl.nsp + pl.ncl - 1;
+            __syncwarp();
+            if (lane == 0) e = pl;
+            __syncwarp();
         }
         if (q != a.q) {  // q is the same on every lane of the warp
             warp_flush(a, acc, ACC_EASY);
@@ -819,7 +828,13 @@ void launch_easy(cpx_ctx *ctx, const Plan &pl)
     CPX_LAUNCH("k_easy_count");
     note_launch(ctx);
     scan_u64(ctx, off, pl.n_easy + 1);
-    const unsigned grid = (unsigned)ctx->sm_count * 8;
+    // CTAs an SM: 32, and 96 from 2^20 units on.  A warp's slice of chunks starts
+    // with a search among the units, which few units do not repay; the more
+    // slices, the closer together the chunks that run at the same time lie in the
+    // prime list and the pi table, and the shorter the last ones.  k_easy, ms,
+    // with 8 / 32 / 96 / 256: pi(1e15) (0.1 M units) 0.385 / 0.380 / 0.434 / 0.495,
+    // batch of 4096 (5.5 M) 11.7 / 10.5 / 10.1 / 10.1, pi(1.9e19) 211 / 206 / 202 / 206.
+    const unsigned grid = (unsigned)ctx->sm_count * (pl.n_easy >> 20 ? 96 : 32);
     KSpan ks(ctx, "k_easy");
     if (pl.wide)
         k_easy<u128><<<grid, kThreads, 0, ctx->stream>>>(pl.qd, pl.Q, pl.pre_easy, pl.n_easy, off, tb.P, tb.prm_max,
