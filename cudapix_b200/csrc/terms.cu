@@ -143,7 +143,13 @@ __global__ void __launch_bounds__(kThreads) k_p2_primes(const QD *__restrict__ q
     uint64_t k0 = 0;
     bool fast = false;
     int64_t s = 0;  // this lane's sum for query a.q since the last fold
-    for (uint64_t base = sl.u0; base < sl.u1; base += 32) {
+    // pi(x/p_k) - k + 1; x/p >= p >= 2
+    auto leaf = [&](uint32_t p, uint64_t k) -> int64_t {
+        const uint64_t v = fast ? cpx_quot40_core<uint64_t>((uint64_t)x, xd, p, cpx_rcp_approx(p))
+                                : (uint64_t)cpx_qdiv(x, (uint64_t)p);
+        return (int64_t)cpx_pi_ge2(T, v) - (int64_t)k + 1;
+    };
+    for (uint64_t base = sl.u0; base < sl.u1;) {
         const uint64_t u = base + lane;
         if (u < sl.u1) {
             const uint32_t q = qlookup(qc, pre, Q, u);
@@ -157,12 +163,24 @@ __global__ void __launch_bounds__(kThreads) k_p2_primes(const QD *__restrict__ q
                 fast = ((u128)x >> 53) == 0 && (d.z >> 41) == 0;
                 xd = (double)(uint64_t)x;
             }
-            const uint64_t k = k0 + 1 + (u - qc.lo);
-            const uint32_t p = __ldg(P + k - 1);
-            const uint64_t v = fast ? cpx_quot40_core<uint64_t>((uint64_t)x, xd, p, cpx_rcp_approx(p))
-                                    : (uint64_t)cpx_qdiv(x, (uint64_t)p);
-            s += (int64_t)cpx_pi_ge2(T, v) - (int64_t)k + 1;  // v >= p >= 2
         }
+        // four primes a lane a step while the first lane's query lasts (its
+        // units hold every lane's then): their loads, which bound the kernel,
+        // overlap (batch of 4096 2.40 -> 1.62 ms, pi(1e17) 0.152 -> 0.121)
+        const uint64_t end = min(sl.u1, (uint64_t)__shfl_sync(FULL, qc.hi, 0));
+        if (base + 128 <= end) {
+            uint64_t k = k0 + 1 + (u - qc.lo);
+            for (; base + 128 <= end; base += 128, k += 128) {
+                const uint32_t p0 = __ldg(P + k - 1), p1 = __ldg(P + k + 31), p2 = __ldg(P + k + 63), p3 = __ldg(P + k + 95);
+                s += (leaf(p0, k) + leaf(p1, k + 32)) + (leaf(p2, k + 64) + leaf(p3, k + 96));
+            }
+            continue;
+        }
+        if (u < sl.u1) {
+            const uint64_t k = k0 + 1 + (u - qc.lo);
+            s += leaf(__ldg(P + k - 1), k);
+        }
+        base += 32;
     }
     a.v += s;
     warp_flush(a, acc, ACC_P2);
@@ -783,11 +801,14 @@ void launch_p2(cpx_ctx *ctx, const Plan &pl)
     if (!pl.n_p2) return;
     KSpan ks(ctx, "k_p2");
     if (pl.p2_primes) {
+        // 8 CTAs an SM; 32 from 2^26 primes on (batch of 4096, 5e8 primes: 1.62 and
+        // 1.45 ms; pi(1e17), 1.7e7 primes: 0.121 and 0.129)
+        const unsigned grid = grid_for(ctx, pl.n_p2) * (pl.n_p2 >> 26 ? 4u : 1u);
         if (pl.wide)
-            k_p2_primes<u128><<<grid_for(ctx, pl.n_p2), kThreads, 0, ctx->stream>>>(pl.qd, pl.Q, pl.pre_p2, pl.n_p2,
+            k_p2_primes<u128><<<grid, kThreads, 0, ctx->stream>>>(pl.qd, pl.Q, pl.pre_p2, pl.n_p2,
                                                                                     ctx->tab.P, ctx->tab.T, pl.acc);
         else
-            k_p2_primes<uint64_t><<<grid_for(ctx, pl.n_p2), kThreads, 0, ctx->stream>>>(
+            k_p2_primes<uint64_t><<<grid, kThreads, 0, ctx->stream>>>(
                 pl.qd, pl.Q, pl.pre_p2, pl.n_p2, ctx->tab.P, ctx->tab.T, pl.acc);
     } else if (pl.wide)
         k_p2<u128><<<grid_for(ctx, pl.n_p2), kThreads, 0, ctx->stream>>>(pl.qd, pl.Q, pl.pre_p2, pl.n_p2,
