@@ -6,7 +6,7 @@
 // CUDA events by coordinate descent: the alpha scale (per mille of the
 // reference alpha), the cap of the hard-leaf segment bits with the threads per
 // segment, the alpha scale again, then the candidate threshold of offloaded
-// leaf sets.
+// leaf sets (which a shared sieve alone offloads).
 // Results are exact under every setting; only the time changes.  Two kinds of
 // entries: one per decade of x, tuned on lone queries at the bottom and the
 // geometric middle of the decade (the plain path; used by batches of up to

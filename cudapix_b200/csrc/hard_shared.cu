@@ -10,13 +10,13 @@
 //      phi(lo_w - 1, b - 1), the survivors below each sub-segment (a level's
 //      first sieved segment starts from the pi table: below p_b^2 the
 //      survivors of level b-1 are 1 and the primes from p_b on);
-//  (3) k_hard_shared runs one CTA per (group of up to 32 queries, segment).
-//      Its warps sieve their sub-segments level by level as k_hard does; at
-//      each level the lanes compute the candidate range of one query each
-//      (from a per-(group, level) table of x/p, y/p and x/p^3 that
-//      k_group_levels fills once per batch), answer their own query's leaves
-//      when every query has few, or else the warp gathers the leaves of every
-//      query and answers them 32 at a time; each leaf's -mu(m) phi(u, b-1) =
+//  (3) k_hard_shared's CTAs take units, a segment and up to 8 groups of up to
+//      32 queries, from a counter.  Its warps sieve their sub-segments level by
+//      level; at each level, group after group, the lanes compute the candidate
+//      range of one query each (from a per-(group, level) table of x/p, y/p and
+//      x/p^3 that k_group_levels fills once per batch) and either answer their
+//      own query's leaves or, when the queries' leaves differ much in number,
+//      the warp takes all of them as one sequence, 32 at a time; each leaf's -mu(m) phi(u, b-1) =
 //      -mu(m) (carry + survivors of the sub-segment <= u) goes straight into
 //      its query's sum: no per-segment outputs and no carry combine.
 // Heavy (query, sub-segment, level) leaf sets go to k_hard_leaves with one

@@ -466,7 +466,8 @@ __global__ void __launch_bounds__(kThreads, 4) k_easy(const QD *__restrict__ qd,
     // plan in shared memory, so that its eighteen registers hold leaves instead
     // (spilled before: k_easy of pi(1.9e19) 259 -> 211 ms, pi(1e17) 7.0 -> 6.7; 48
     // or 40 registers a thread and more warps: 219 and 218, 6.6 and 6.45, and 12.1
-    // and 12.2 ms on the batch of 4096 where 64 registers take 11.7)
+    // and 12.2 ms on the batch of 4096 where 64 registers take 11.7); one lane
+    // unpacks it there (10.1 -> 9.7 ms on the batch against a copy from each lane's)
     __shared__ EasyP s_e[kThreads / 32];
     EasyP &e = s_e[threadIdx.x >> 5];
     uint64_t c_unit = ~0ull, c_first = 0, c_last = 0, b = 0;
@@ -488,11 +489,11 @@ __global__ void __launch_bounds__(kThreads, 4) k_easy(const QD *__restrict__ qd,
                 do c_unit++;
                 while (__ldg(off + c_unit + 1) <= ch);
             }
-            EasyP pl = {};
+            __syncwarp();  // the chunk before has been read
             if (rec) {
                 const EasyRec r = rec[c_unit];
                 xp = (XT)r.xp;
-                easy_unpack(r, pl);
+                if (lane == 0) easy_unpack(r, e);
                 b = r.b;
                 q = r.q;
             } else {
@@ -500,13 +501,13 @@ __global__ void __launch_bounds__(kThreads, 4) k_easy(const QD *__restrict__ qd,
                 const QD &d = qd[q];
                 const uint64_t i = c_unit - __ldg(pre + q);
                 b = d.c + 1 + i;  // p = p_b
+                EasyP pl = {};
                 easy_plan<XT>(xload<XT>(d), d.y, __ldg(P + d.c + i), prm_max, T, xp, pl);
+                if (lane == 0) e = pl;
             }
+            __syncwarp();
             c_first = __ldg(off + c_unit);
-            c_last = c_first + pl.nsp + pl.ncl - 1;
-            __syncwarp();
-            if (lane == 0) e = pl;
-            __syncwarp();
+            c_last = c_first + e.nsp + e.ncl - 1;
         }
         if (q != a.q) {  // q is the same on every lane of the warp
             warp_flush(a, acc, ACC_EASY);
@@ -657,7 +658,9 @@ __global__ void __launch_bounds__(kThreads) k_easy_comp(const QD *__restrict__ q
 // few are composite with a least factor above the levels' smallest prime pmin
 // (pi(1e17): 7e9 m over 630 levels for 1.6e7 leaves).  k_comp_list writes those
 // down once, {m | (mu(m) = -1) << 31, lpf(m)} in no order, and each level goes
-// through the list: pi(1e17) 4.59 -> 0.24 ms, pi(1.9e19) 18.8 -> 0.44.  cap entries always suffice (the host's bound).
+// through the list: pi(1e17) 4.59 -> 0.24 ms, pi(1.9e19) at the
+// reference alpha 18.8 -> 0.44 (at 3.5 times it, where that call is fastest, the
+// list is longer: 19).  cap entries always suffice (the host's bound).
 __global__ void __launch_bounds__(kThreads) k_comp_list(const int32_t *__restrict__ MU, uint64_t i_lo, uint64_t i_hi,
                                                         uint32_t pmin, uint32_t cap, uint2 *__restrict__ list,
                                                         unsigned int *__restrict__ count)
